@@ -132,6 +132,13 @@ int qsdvr_ray_cut(const qsdvr_camera *camera, const uint8_t *mask, qsdvr_ray_inf
 int qsdvr_ray_cut_noalloc(const qsdvr_camera *camera, const uint8_t *mask, qsdvr_ray_info *rays, float *origin,
                           float *dir, float interval, uint32_t pixel_count, uint32_t *totals, cudaStream_t stream);
 
+/* The rays of the listed pixels, out_*[i] = *[pixels[i]] for i < count: what a camera keeps of
+ * qsdvr_ray_cut's per-pixel tables after masking (datasets/utils.py:50-56 indexes three tensors).
+ * A pixel outside [0, pixel_count) gives a zero ray and sets QSDVR_DEVERR_INDEX. */
+int qsdvr_gather_rays(const int64_t *pixels, uint32_t count, uint32_t pixel_count, const qsdvr_ray_info *rays,
+                      const float *origin, const float *dir, qsdvr_ray_info *out_rays, float *out_origin,
+                      float *out_dir, cudaStream_t stream);
+
 /* Replaces GenerateRayPoints (kernel/camera.cu:132-147, include/camera.h:59).
  * sdf_capacity / render_capacity are the lengths of the sample lists. */
 int qsdvr_generate_ray_points(const qsdvr_ray_info *rays, const float *origin, const float *dir,

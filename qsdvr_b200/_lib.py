@@ -46,6 +46,7 @@ _SIGS = {
     "qsdvr_bounds_record": [P, I32, P],
     "qsdvr_check_bounds": [P, P],
     "qsdvr_ray_cut": [ctypes.POINTER(Camera), P, P, P, P, F32, U32, P, P, SZ, P],
+    "qsdvr_gather_rays": [P, U32, U32, P, P, P, P, P, P, P],
     "qsdvr_generate_ray_points": [P, P, P, U32, F32, U32, P, P, P, P, P, U64, U64, P],
     "qsdvr_layer_to_grid_forward": [P, P, P, P, P, U32, P, SZ, P],
     "qsdvr_layer_to_grid_backward": [P, U32, P, P, P, P, P, SZ, P],

@@ -7,13 +7,14 @@ tables to the host after RayCut and back on every call).
 """
 from __future__ import annotations
 
+import ctypes
 import struct
 import zlib
 
 import numpy as np
 import torch
 
-from . import qsdvr
+from . import _lib, qsdvr
 from .qsdvr import CameraArgs
 
 
@@ -56,18 +57,18 @@ class Camera:
         dev = self.device
         P = self.args.pixelCount
         rays = torch.zeros((P, 4), dtype=torch.int32, device=dev)
-        origin = torch.zeros((P, 3), dtype=torch.float32, device=dev)
-        direction = torch.zeros((P, 3), dtype=torch.float32, device=dev)
-        qsdvr.RayCut(self.args, mask, rays, origin, direction, self.interval)
+        origin = torch.empty((P, 3), dtype=torch.float32, device=dev)  # RayCut writes every pixel's
+        direction = torch.empty((P, 3), dtype=torch.float32, device=dev)
         m = mask.reshape(-1)[:P].to(dev, torch.bool)
+        # a boolean mask crosses to the device once
+        qsdvr.RayCut(self.args, m if mask.dtype == torch.bool and m.numel() == P else mask, rays, origin, direction,
+                     self.interval)
         self.mask = m
         pix = torch.nonzero(m).reshape(-1)
         if order == "tiles":
             pix = tile_order(pix, self.args.width, tile)
         self.pixel_index = pix
-        self.rayList = rays[pix].contiguous()
-        self.originList = origin[pix].contiguous()
-        self.dirList = direction[pix].contiguous()
+        self.rayList, self.originList, self.dirList = gather_rays(pix, rays, origin, direction)
 
     def whole_image(self, colors: torch.Tensor) -> torch.Tensor:
         """datasets/nerf_dataset.py:92-96 (get_whole_image): the rays' colours [N, 3] (in the
@@ -80,6 +81,18 @@ class Camera:
         img = torch.zeros((a.height * a.width, 3), dtype=colors.dtype, device=colors.device)
         img[pix] = colors
         return img.reshape(a.height, a.width, 3)
+
+
+def gather_rays(pixels: torch.Tensor, rays, origin, direction):
+    """(rays, origin, direction) of the listed pixels (int64 indices), one launch."""
+    n, dev = pixels.numel(), rays.device
+    out = (torch.empty((n, 4), dtype=torch.int32, device=dev), torch.empty((n, 3), dtype=torch.float32, device=dev),
+           torch.empty((n, 3), dtype=torch.float32, device=dev))
+    with torch.cuda.device(dev):
+        _lib.call("qsdvr_gather_rays", ctypes.c_void_p(pixels.data_ptr()), n, rays.shape[0],
+                  *(ctypes.c_void_p(t.data_ptr()) for t in (rays, origin, direction, *out)),
+                  ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream))
+    return out
 
 
 def tile_order(pixels: torch.Tensor, width: int, tile: int = 8) -> torch.Tensor:

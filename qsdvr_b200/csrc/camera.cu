@@ -33,8 +33,39 @@ __device__ __forceinline__ f3 camera_to_world(const qsdvr_camera &c, float px, f
     return w;
 }
 
+constexpr float kBox = 0.9999f;  // the in-box test is strict: |x|, |y|, |z| < kBox
+
 __device__ __forceinline__ bool in_box(float x, float y, float z) {
-    return x < 0.9999f && x > -0.9999f && y < 0.9999f && y > -0.9999f && z < 0.9999f && z > -0.9999f;
+    return x < kBox && x > -kBox && y < kBox && y > -kBox && z < kBox && z > -kBox;
+}
+
+// First j in [0, n] for which pred holds, for a pred that stays true once it is (n if never).
+template <typename Pred>
+__device__ __forceinline__ uint32_t first_true(uint32_t n, Pred pred) {
+    uint32_t lo = 0;
+    while (lo < n) {
+        const uint32_t mid = (lo + n) >> 1;
+        if (pred(mid)) n = mid;
+        else lo = mid + 1;
+    }
+    return lo;
+}
+
+// The march samples j in [0, steps) whose coordinate n + (d j) interval lies inside the box: [a, b).
+// Rounding is monotone, so the float32 coordinate of sample j is monotone in j and the run's ends
+// are found by bisection on the very values the march produces (d finite).
+__device__ __forceinline__ void axis_run(float n, float d, float interval, uint32_t steps, uint32_t &a, uint32_t &b) {
+    auto at = [&](uint32_t j) { return __fmaf_rn(__fmul_rn(d, (float)j), interval, n); };
+    if (d > 0.0f) {
+        a = first_true(steps, [&](uint32_t j) { return at(j) > -kBox; });
+        b = first_true(steps, [&](uint32_t j) { return !(at(j) < kBox); });
+    } else if (d < 0.0f) {
+        a = first_true(steps, [&](uint32_t j) { return at(j) < kBox; });
+        b = first_true(steps, [&](uint32_t j) { return !(at(j) > -kBox); });
+    } else {
+        a = 0;
+        b = n < kBox && n > -kBox ? steps : 0;
+    }
 }
 
 // Masked (sdf, render) contribution of a pixel with raw in-box count c (kernel/camera.cu:115-126).
@@ -114,17 +145,30 @@ __global__ void __launch_bounds__(kScanBlock) ray_cut_kernel(qsdvr_camera cam, f
             flag_error(QSDVR_DEVERR_RAY);
             steps = 0;
         }
-        // The in-box samples form one contiguous run of j (each coordinate is monotone in
-        // j), so the march stops at the first sample that leaves the box after entering.
+        // The in-box samples form one contiguous run of j (each coordinate is monotone in j):
+        // the intersection of the axes' runs, each found by bisection, instead of a march through
+        // up to `steps` samples (512 at 512 samples a ray: 251 -> 22 us for an 800 x 800 view).
         uint32_t hits = 0;
         f3 first{0.0f, 0.0f, 0.0f};
-        for (uint32_t j = 0; j < steps; ++j) {
-            const f3 p = march(n, d, (float)j, interval);
-            if (in_box(p.x, p.y, p.z)) {
-                if (hits == 0) first = p;
-                ++hits;
-            } else if (hits) {
-                break;
+        if (isfinite(d.x) && isfinite(d.y) && isfinite(d.z)) {
+            uint32_t ax, bx, ay, by, az, bz;
+            axis_run(n.x, d.x, interval, steps, ax, bx);
+            axis_run(n.y, d.y, interval, steps, ay, by);
+            axis_run(n.z, d.z, interval, steps, az, bz);
+            const uint32_t lo = max(ax, max(ay, az)), hi = min(bx, min(by, bz));
+            if (lo < hi) {
+                hits = hi - lo;
+                first = march(n, d, (float)lo, interval);
+            }
+        } else {
+            for (uint32_t j = 0; j < steps; ++j) {
+                const f3 p = march(n, d, (float)j, interval);
+                if (in_box(p.x, p.y, p.z)) {
+                    if (hits == 0) first = p;
+                    ++hits;
+                } else if (hits) {
+                    break;
+                }
             }
         }
         store3(dir + 3ull * id, d);
@@ -180,6 +224,31 @@ __global__ void __launch_bounds__(kScanBlock) ray_cut_apply_kernel(uint32_t pixe
         r.render_offset = base.y + ex.y;
         rays[id] = r;
     }
+}
+
+// The rays of the listed pixels (Camera keeps the masked ones): record, origin and direction in
+// one pass, a thread per ray.  Three generic row gathers took 370 us for an 800 x 800 view (331 of
+// them for the 16-byte records); 7 us now.
+__global__ void __launch_bounds__(256) gather_rays_kernel(const int64_t *__restrict__ pixels, uint32_t count,
+                                                          uint32_t pixel_count,
+                                                          const qsdvr_ray_info *__restrict__ rays,
+                                                          const float *__restrict__ origin,
+                                                          const float *__restrict__ dir,
+                                                          qsdvr_ray_info *__restrict__ out_rays,
+                                                          float *__restrict__ out_origin, float *__restrict__ out_dir) {
+    const uint32_t i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= count) return;
+    const int64_t p = pixels[i];
+    if (p < 0 || p >= (int64_t)pixel_count) {
+        flag_error(QSDVR_DEVERR_INDEX);
+        reinterpret_cast<uint4 *>(out_rays)[i] = make_uint4(0, 0, 0, 0);
+        store3(out_origin + 3ull * i, f3{0.0f, 0.0f, 0.0f});
+        store3(out_dir + 3ull * i, f3{0.0f, 0.0f, 0.0f});
+        return;
+    }
+    reinterpret_cast<uint4 *>(out_rays)[i] = reinterpret_cast<const uint4 *>(rays)[p];
+    store3(out_origin + 3ull * i, load3(origin + 3 * p));
+    store3(out_dir + 3ull * i, load3(dir + 3 * p));
 }
 
 // kernel/camera.cu:60-96 — one warp per ray, lanes stride over the ray's samples so the
@@ -247,6 +316,19 @@ extern "C" int qsdvr_ray_cut(const qsdvr_camera *camera, const uint8_t *mask, qs
     scan_block_sums_kernel<<<1, 1024, 0, stream>>>(sums, blocks, totals);
     ray_cut_apply_kernel<<<blocks, kScanBlock, 0, stream>>>(pixel_count, mask, rays, sums);
     return check_launch("qsdvr_ray_cut");
+}
+
+extern "C" int qsdvr_gather_rays(const int64_t *pixels, uint32_t count, uint32_t pixel_count,
+                                 const qsdvr_ray_info *rays, const float *origin, const float *dir,
+                                 qsdvr_ray_info *out_rays, float *out_origin, float *out_dir, cudaStream_t stream) {
+    if (count == 0) return QSDVR_OK;
+    if (!pixels || !rays || !origin || !dir || !out_rays || !out_origin || !out_dir)
+        return set_error(QSDVR_ERR_INVALID_ARGUMENT, "qsdvr_gather_rays: null pointer");
+    if (!aligned(rays, 16) || !aligned(out_rays, 16) || !aligned(pixels, 8))
+        return set_error(QSDVR_ERR_ALIGNMENT, "qsdvr_gather_rays: rays need 16-byte, pixels 8-byte alignment");
+    gather_rays_kernel<<<grid_for(count, 256), 256, 0, stream>>>(pixels, count, pixel_count, rays, origin, dir, out_rays,
+                                                                 out_origin, out_dir);
+    return check_launch("qsdvr_gather_rays");
 }
 
 extern "C" int qsdvr_generate_ray_points(const qsdvr_ray_info *rays, const float *origin, const float *dir,
