@@ -42,6 +42,9 @@ namespace {
 #ifndef QSDVR_FUSED_MIN_BLOCKS
 #define QSDVR_FUSED_MIN_BLOCKS 16
 #endif
+#ifndef QSDVR_FORWARD_MIN_BLOCKS
+#define QSDVR_FORWARD_MIN_BLOCKS 20
+#endif
 #ifndef QSDVR_GATHER_UNROLL
 #define QSDVR_GATHER_UNROLL 2
 #endif
@@ -64,8 +67,13 @@ constexpr uint32_t kMaxChunks = 256;  // render samples per ray <= 8192
 // sample's (base vertex, wx, wy, wz), the vertex kNoVertex for a sample without a row, so a
 // step reads one sample's parameters with one 16-byte shared load instead of 5 shuffles.
 constexpr uint32_t kNoVertex = 0xffffffffu;
+constexpr uint32_t kLossParts = 32;  // word offset of the loss's partial sums behind the ray counter
 
 enum Pass { kForward = 0, kBackward = 1, kTrain = 2 };
+// Resident one-warp blocks per SM that each pass is compiled for.  The forward's 20 are what its
+// shared memory allows; compiled for 16 it took up to 126 registers and lost four of them (a 384^3
+// frame 7.0 instead of 6.0 ms).
+constexpr int min_blocks(int pass) { return pass == kForward ? QSDVR_FORWARD_MIN_BLOCKS : QSDVR_FUSED_MIN_BLOCKS; }
 
 // Persistent train mode: each warp stashes the interpolated rows of the kSlotChunks chunks
 // before a ray's last one (the last stays in shared memory) so that the backward reloads
@@ -130,7 +138,8 @@ struct Params {
     float *data_grad;
     float *loss;
     float grad_scale;
-    uint32_t *ray_counter;  // persistent mode: next ray to take (zeroed before the launch)
+    uint32_t *ray_counter;  // persistent mode: next ray to take (zeroed before the launch), then
+                            // in train mode the warps that are done and the loss's partial sums
     float *slots;           // persistent train mode: per-warp row stash, kSlotChunks chunks each
     const float *tlist;     // list sampling: per ray kListT SDF positions (t from origin), or null
     float *sample_alpha;    // optional per-render-sample alpha output (forward, train)
@@ -167,8 +176,9 @@ struct Store<float> {
         a[0] = lo.x; a[1] = lo.y; a[2] = lo.z; a[3] = lo.w;
         a[4] = hi.x; a[5] = hi.y; a[6] = hi.z;
     }
-    __device__ static float4 quad(const void *d, uint32_t v, int q, int C, uint64_t verts) {
-        return ld4(QSDVR_AT(static_cast<const float *>(d), (uint64_t)C * v + 4 * q, 4, (uint64_t)C * verts));
+    // elements [e, e + 4) of the appearance grid: one 16-byte load
+    __device__ static float4 quad(const void *d, uint64_t e, [[maybe_unused]] uint64_t extent) {
+        return ld4(QSDVR_AT(static_cast<const float *>(d), e, 4, extent));
     }
 };
 
@@ -182,10 +192,9 @@ struct Store<__nv_bfloat16> {
         // into two bf16; exact in fp32)
         a[4] = bf_lo(r.z); a[5] = bf_hi(r.z); a[6] = bf_lo(r.w) + bf_hi(r.w);
     }
-    // channels [8q, 8q + 8) of vertex v: one 16-byte load (bf16 x 8)
-    __device__ static uint4 oct(const void *d, uint32_t v, int q, int C, uint64_t verts) {
-        return *reinterpret_cast<const uint4 *>(
-            QSDVR_AT(static_cast<const __nv_bfloat16 *>(d), (uint64_t)C * v + 8 * q, 8, (uint64_t)C * verts));
+    // elements [e, e + 8) of the appearance grid: one 16-byte load (bf16 x 8)
+    __device__ static uint4 oct(const void *d, uint64_t e, [[maybe_unused]] uint64_t extent) {
+        return *reinterpret_cast<const uint4 *>(QSDVR_AT(static_cast<const __nv_bfloat16 *>(d), e, 8, extent));
     }
 };
 
@@ -395,65 +404,109 @@ struct Sample {
     float wx, wy, wz;
 };
 
+// What a chunk's first lane needs of the SDF sample before the chunk's own: its alpha term,
+// whether its cell lies in the grid (bit 0) and whether it is finite (bit 1).  The last lane of
+// one chunk hands it to the next, so each SDF sample and its alpha term are evaluated once:
+// evaluating the chunk's first sample on lane 0 alone cost the whole warp a pass through the cell
+// evaluation per chunk, a tenth of the instructions of the frame forward, which issue bounds
+// (71 % of the issue slots).  With it, with rows only for the samples that are shaded (unshaded
+// ones were staged, stashed and reloaded as zeros) and with chunks that shade nothing leaving
+// early: 384^3 frame 6.74 -> 5.95 ms, its proposal form 1.82 -> 1.79; train at 256^3 fp32 degree 2
+// 1.62 -> 1.58 ms, bf16 degree 3 2.35 -> 2.19 ms.
+struct Edge {
+    float e;
+    uint32_t bits;
+};
+
+template <bool kCompat>
+__device__ __forceinline__ uint32_t edge_bits(float sdf) {
+    return kCompat || isfinite(sdf) ? 3u : 1u;
+}
+
+// SDF sample 0 of a ray.
+template <bool kCompat, typename S, int kVar>
+__device__ __forceinline__ Edge first_edge(const Params &p, uint32_t r, f3 o, f3 d) {
+    const CellPoint c0 =
+        to_cell(p.tlist ? at_t(o, d, *QSDVR_AT(p.tlist, (uint64_t)kListT * r, kListT, (uint64_t)kListT * p.n))
+                        : march(o, d, 0.0f, p.interval),
+                p.volume_offset, p.R);
+    float s0 = 0.0f;
+    Edge edge{0.0f, 0u};
+    if (cell_in_grid(c0, p.R)) {
+        float a0[7];
+        load_cell<S, kVar>(p, c0, a0);
+        s0 = checked_sdf<kCompat>(a0, c0.u, (float)p.R);
+        edge.bits = edge_bits<kCompat>(s0);
+    }
+    edge.e = alpha_term<kCompat>(p.k, s0);
+    return edge;
+}
+
+// The alpha terms of the chunk's intervals from each lane's own SDF sample i+1 (s1, with its
+// bits) and the edge before the chunk; replaces the edge by the one after it.  Returns the bits
+// of both ends and-ed.
+template <bool kCompat>
+__device__ __forceinline__ uint32_t chunk_terms(const Params &p, float s1, uint32_t b1, int lane, Edge &edge,
+                                                float &e0, float &e1) {
+    e1 = alpha_term<kCompat>(p.k, s1);
+    e0 = __shfl_up_sync(kFull, e1, 1);
+    uint32_t b0 = __shfl_up_sync(kFull, b1, 1);
+    if (lane == 0) {
+        e0 = edge.e;
+        b0 = edge.bits;
+    }
+    edge.e = __shfl_sync(kFull, e1, kWarp - 1);
+    edge.bits = __shfl_sync(kFull, b1, kWarp - 1);
+    return b0 & b1;
+}
+
 // Forward evaluation of render sample i = chunk*32 + lane (kernel/camera.cu:60-96,
-// kernel/surface.cu:54-115, kernel/render.cu:98-179, :239-244).  Leaves the sample's
-// interpolated 32 channels in the warp's tile.
+// kernel/surface.cu:54-115, kernel/render.cu:98-179, :239-244).  Leaves the interpolated
+// channels of the shaded samples in their rows of the warp's tile (the other rows are not
+// written: nothing reads them).
 template <bool kCompat, typename S, int kDeg, int kVar>
 __device__ __forceinline__ void eval_chunk(const Params &p, uint32_t r, f3 o, f3 d, uint32_t nr, uint32_t chunk,
-                                           int lane, float *tile, Sample &s, const float *from_slot = nullptr,
-                                           float *to_slot = nullptr) {
+                                           int lane, float *tile, Sample &s, Edge &edge,
+                                           const float *from_slot = nullptr, float *to_slot = nullptr) {
     using RW = Rows<kDeg>;
     constexpr int kC = RW::kC, kRow = RW::kStride, kL = RW::kLanes, kPS = RW::kPerStep;
     const uint32_t R = p.R;
     const uint32_t i = chunk * kWarp + lane;
     const bool live = i < nr;
-    bool ok = live;
     const float *tl = p.tlist ? QSDVR_AT(p.tlist, (uint64_t)kListT * r, kListT, (uint64_t)kListT * p.n) : nullptr;
     // SDF sample i+1 (this lane's interval end); sample i comes from the previous lane.
     s.c1 = to_cell(tl ? at_t(o, d, live ? tl[i + 1] : 0.0f) : march(o, d, (float)(i + 1), p.interval),
                    p.volume_offset, R);
-    float a1[7];
-    float s1 = 0.0f;
-    if (live) {
-        if (cell_in_grid(s.c1, R)) {
-            load_cell<S, kVar>(p, s.c1, a1);
-            s1 = checked_sdf<kCompat>(a1, s.c1.u, (float)R);
-        } else {
-            ok = false;
-        }
-    }
-    float s0 = __shfl_up_sync(kFull, s1, 1);
-    if (lane == 0 && live) {
-        const CellPoint c0 =
-            to_cell(tl ? at_t(o, d, tl[i]) : march(o, d, (float)i, p.interval), p.volume_offset, R);
-        if (cell_in_grid(c0, R)) {
-            float a0[7];
-            load_cell<S, kVar>(p, c0, a0);
-            s0 = checked_sdf<kCompat>(a0, c0.u, (float)R);
-        } else {
-            ok = false;
-        }
-    }
-    const bool ok_prev = __shfl_up_sync(kFull, ok, 1);
-    if (lane > 0) ok = ok && ok_prev;  // sdf_i is only valid if the previous lane's cell was
-    // render sample i
+    // render sample i; its cell is asked into L2 while the end point's is loaded and evaluated
     s.cr = to_cell(tl ? at_t(o, d, live ? 0.5f * (tl[i] + tl[i + 1]) : 0.0f) : midpoint(o, d, i, p.interval),
                    p.volume_offset, R);
+    const bool in_cr = live && cell_in_grid(s.cr, R);
+    if ((kVar & kVarSep) == 0 && in_cr)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(
+            QSDVR_AT(static_cast<const S *>(p.sdf), 8ull * (uint32_t)s.cr.index, 8, 8ull * R * R * R)));
+    float a1[7];
+    float s1 = 0.0f;
+    uint32_t b1 = 0;
+    if (live && cell_in_grid(s.c1, R)) {
+        load_cell<S, kVar>(p, s.c1, a1);
+        s1 = checked_sdf<kCompat>(a1, s.c1.u, (float)R);
+        b1 = edge_bits<kCompat>(s1);
+    }
     float ar[7];
-    if (live && cell_in_grid(s.cr, R)) {
+    bool ok = in_cr;
+    if (ok) {
         load_cell<S, kVar>(p, s.cr, ar);
         s.nrm = sample_normal<kCompat>(ar, s.cr.u);
     } else {
-        ok = false;
         s.nrm = f3{0.0f, 0.0f, 1.0f};
     }
-    if (live && !ok) flag_error(QSDVR_DEVERR_INDEX);
-    // fixed mode: a sample whose first-order distance is not finite (|grad f| = 0 in a cell)
-    // is empty; compat keeps the reference's arithmetic, non-finite values included
-    if (!kCompat && !(isfinite(s0) && isfinite(s1))) ok = false;
+    // an interval is valid if its render sample's cell and both ends' cells are in the grid; fixed
+    // mode: a sample whose first-order distance is not finite (|grad f| = 0 in a cell) is empty;
+    // compat keeps the reference's arithmetic, non-finite values included
+    const uint32_t bits = chunk_terms<kCompat>(p, s1, b1, lane, edge, s.e0, s.e1);
+    if (live && !(ok && (bits & 1u))) flag_error(QSDVR_DEVERR_INDEX);
+    ok = ok && bits == 3u;
     s.valid = ok;
-    s.e0 = alpha_term<kCompat>(p.k, s0);
-    s.e1 = alpha_term<kCompat>(p.k, s1);
     s.alpha = ok ? interval_alpha<kCompat>(s.e0, s.e1) : 0.0f;
     // A valid sample with alpha = 0 (the SDF does not fall across its interval: about half
     // of a ray's samples) adds alpha T c = 0 to the colour, and every backward term of its
@@ -462,6 +515,9 @@ __device__ __forceinline__ void eval_chunk(const Params &p, uint32_t r, f3 o, f3
     // appearance rows.  A non-finite normal keeps the full path, so the NaN colour of a
     // degenerate cell propagates as in the reference.
     s.shaded = ok && (s.alpha != 0.0f || !(isfinite(s.nrm.x) && isfinite(s.nrm.y) && isfinite(s.nrm.z)));
+    const uint32_t shaded = __ballot_sync(kFull, s.shaded);
+    s.rgb = f3{0.0f, 0.0f, 0.0f};
+    s.spec = f3{0.0f, 0.0f, 0.0f};
     // trilinear weights and base vertex (kernel/render.cu:107-111)
     s.wx = (s.cr.u.x + 1.0f) / 2.0f;
     s.wy = (s.cr.u.y + 1.0f) / 2.0f;
@@ -469,6 +525,7 @@ __device__ __forceinline__ void eval_chunk(const Params &p, uint32_t r, f3 o, f3
     const uint32_t R1 = R + 1;
     s.vbase = kCompat ? (uint32_t)s.cr.index
                       : (uint32_t)s.cr.cx + (uint32_t)s.cr.cy * R1 + (uint32_t)s.cr.cz * (R1 * R1);
+    if (shaded == 0) return;  // no sample of the chunk has a colour
     const int q = lane % kL;
     const uint32_t sy = R1, sz = R1 * R1;
     [[maybe_unused]] const uint64_t nv = (uint64_t)R1 * R1 * R1;  // vertex rows
@@ -486,10 +543,6 @@ __device__ __forceinline__ void eval_chunk(const Params &p, uint32_t r, f3 o, f3
         }
     }
 #endif
-    if (!from_slot) {
-        st4(tile + lane * kRow + kC, make_float4(__uint_as_float(s.shaded ? s.vbase : kNoVertex), s.wx, s.wy, s.wz));
-        __syncwarp();
-    }
     if (from_slot) {
         // rows stashed by the forward, one row per kL lanes per step, copied into the tile by
         // asynchronous 16-byte copies that are all in flight at once (one L2 round trip per
@@ -498,155 +551,124 @@ __device__ __forceinline__ void eval_chunk(const Params &p, uint32_t r, f3 o, f3
 #pragma unroll
         for (int st = 0; st < kL; ++st) {
             const int j = st * kPS + lane / kL;
-            cp_async16_keep(tile + j * kRow + 4 * q, from_slot + j * kC + 4 * q, pol);
+            if ((shaded >> j) & 1u) cp_async16_keep(tile + j * kRow + 4 * q, from_slot + j * kC + 4 * q, pol);
         }
         cp_async_wait();
+        __syncwarp();
 #if QSDVR_STASH_DISCARD
         // The stash is dead once read: drop its L2 lines without writing them back (they
         // would otherwise reach DRAM as dirty evictions) and free the room for the gathers.
         // Every lane's copies have completed (cp.async.wait_all before the warp barrier).
-        __syncwarp();
-        constexpr uint32_t kLines = kWarp * kC * sizeof(float) / 128;  // the chunk's 128-byte lines
-        for (uint32_t l = lane; l < kLines; l += kWarp)
-            asm volatile("discard.global.L2 [%0], 128;" ::"l"(from_slot + l * (128 / sizeof(float))) : "memory");
-#endif
-    } else if constexpr (sizeof(S) == 2) {
-        // bf16 storage: groups of kGL lanes fetch one sample's 8 corner rows as 16-byte
-        // (bf16 x 8) loads, kGPS samples per step; each lane stages 8 interpolated channels
-        using GL = GatherLanes<S, kDeg>;
-        constexpr int kGL = GL::kLanes, kGPS = GL::kPerStep;
-        const int q8 = lane % kGL;
-#pragma unroll kGatherUnroll
-        for (int st = 0; st < kGL; ++st) {
-            const int j = st * kGPS + lane / kGL;
-            const float4 prm = ld4(tile + j * kRow + kC);
-            const uint32_t vb = __float_as_uint(prm.x);
-            const float gx = prm.y, gy = prm.z, gz = prm.w;
-            const bool gok = vb != kNoVertex;
-            float v[8];
-            if (gok) {
-                const uint4 v000 = Store<S>::oct(p.data, vb, q8, kC, nv), v001 = Store<S>::oct(p.data, vb + 1, q8, kC, nv);
-                const uint4 v010 = Store<S>::oct(p.data, vb + sy, q8, kC, nv),
-                            v011 = Store<S>::oct(p.data, vb + sy + 1, q8, kC, nv);
-                const uint4 v100 = Store<S>::oct(p.data, vb + sz, q8, kC, nv),
-                            v101 = Store<S>::oct(p.data, vb + sz + 1, q8, kC, nv);
-                const uint4 v110 = Store<S>::oct(p.data, vb + sz + sy, q8, kC, nv),
-                            v111 = Store<S>::oct(p.data, vb + sz + sy + 1, q8, kC, nv);
-                float w[8];
-                corner_weights(gx, gy, gz, w);
-                first_bf8(v000, w[0], v);
-                fma_bf8(v001, w[1], v);
-                fma_bf8(v010, w[2], v);
-                fma_bf8(v011, w[3], v);
-                fma_bf8(v100, w[4], v);
-                fma_bf8(v101, w[5], v);
-                fma_bf8(v110, w[6], v);
-                fma_bf8(v111, w[7], v);
-            } else {
+        if (s.shaded) {
 #pragma unroll
-                for (int t = 0; t < 8; ++t) v[t] = 0.0f;
-            }
-            const float4 lo = make_float4(v[0], v[1], v[2], v[3]), hi = make_float4(v[4], v[5], v[6], v[7]);
-            // with 8 lanes per row (64 channels) lanes 4..7 store their halves in the other
-            // order, so each 8-lane phase of a store covers 32 distinct banks
-            const bool swap = (q8 & 4) != 0;
-            st4(tile + j * kRow + 8 * q8 + (swap ? 4 : 0), swap ? hi : lo);
-            st4(tile + j * kRow + 8 * q8 + (swap ? 0 : 4), swap ? lo : hi);
-            if (to_slot) {
-                const uint64_t pol = evict_last_policy();
-                st4_keep(to_slot + j * kC + 8 * q8, lo, pol);
-                st4_keep(to_slot + j * kC + 8 * q8 + 4, hi, pol);
-            }
+            for (int l = 0; l < kC * 4 / 128; ++l)  // the row's 128-byte lines
+                asm volatile("discard.global.L2 [%0], 128;" ::"l"(from_slot + lane * kC + l * 32) : "memory");
         }
+#endif
     } else {
-    // gather: groups of kL lanes fetch one sample's 8 corner rows, kPS samples per step
-#pragma unroll kGatherUnroll
-    for (int st = 0; st < kL; ++st) {
-        const int j = st * kPS + lane / kL;
-        const float4 prm = ld4(tile + j * kRow + kC);
-        const uint32_t vb = __float_as_uint(prm.x);
-        const float gx = prm.y, gy = prm.z, gz = prm.w;
-        const bool gok = vb != kNoVertex;
-        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (gok) {
-            const float4 v000 = Store<S>::quad(p.data, vb, q, kC, nv), v001 = Store<S>::quad(p.data, vb + 1, q, kC, nv);
-            const float4 v010 = Store<S>::quad(p.data, vb + sy, q, kC, nv),
-                         v011 = Store<S>::quad(p.data, vb + sy + 1, q, kC, nv);
-            const float4 v100 = Store<S>::quad(p.data, vb + sz, q, kC, nv),
-                         v101 = Store<S>::quad(p.data, vb + sz + 1, q, kC, nv);
-            const float4 v110 = Store<S>::quad(p.data, vb + sz + sy, q, kC, nv),
-                         v111 = Store<S>::quad(p.data, vb + sz + sy + 1, q, kC, nv);
-            float w[8];
-            corner_weights(gx, gy, gz, w);
-            v = scale4(v000, w[0]);
-            fma4(v, v001, w[1]);
-            fma4(v, v010, w[2]);
-            fma4(v, v011, w[3]);
-            fma4(v, v100, w[4]);
-            fma4(v, v101, w[5]);
-            fma4(v, v110, w[6]);
-            fma4(v, v111, w[7]);
+        st4(tile + lane * kRow + kC, make_float4(__uint_as_float(s.shaded ? s.vbase : kNoVertex), s.wx, s.wy, s.wz));
+        __syncwarp();
+        // Groups of kGL lanes fetch one sample's 8 corner rows (16 bytes a lane and corner), kGPS
+        // samples per step, kGatherUnroll steps at a time; samples without a colour are skipped.
+        using GL = GatherLanes<S, kDeg>;
+        constexpr int kGL = GL::kLanes, kGPS = GL::kPerStep, kCh = GL::kCh, kRound = kGPS * kGatherUnroll;
+        constexpr uint32_t kRoundMask = kRound >= 32 ? 0xffffffffu : (1u << (kRound & 31)) - 1u;
+        const uint64_t dy = (uint64_t)kC * sy, dz = (uint64_t)kC * sz, ne = nv * kC;  // in elements
+        const int gq = lane % kGL;
+#pragma unroll 1
+        for (int first = 0; first < kWarp; first += kRound) {
+            if (((shaded >> first) & kRoundMask) == 0) continue;  // warp-uniform
+#pragma unroll
+            for (int u = 0; u < kGatherUnroll; ++u) {
+                const int j = first + u * kGPS + lane / kGL;
+                const float4 prm = ld4(tile + j * kRow + kC);
+                const uint32_t vb = __float_as_uint(prm.x);
+                if (vb == kNoVertex) continue;
+                const uint64_t e = (uint64_t)kC * vb + kCh * gq;
+                float w[8];
+                corner_weights(prm.y, prm.z, prm.w, w);
+                if constexpr (sizeof(S) == 2) {
+                    const uint4 v000 = Store<S>::oct(p.data, e, ne), v001 = Store<S>::oct(p.data, e + kC, ne);
+                    const uint4 v010 = Store<S>::oct(p.data, e + dy, ne),
+                                v011 = Store<S>::oct(p.data, e + dy + kC, ne);
+                    const uint4 v100 = Store<S>::oct(p.data, e + dz, ne),
+                                v101 = Store<S>::oct(p.data, e + dz + kC, ne);
+                    const uint4 v110 = Store<S>::oct(p.data, e + dz + dy, ne),
+                                v111 = Store<S>::oct(p.data, e + dz + dy + kC, ne);
+                    float v[8];
+                    first_bf8(v000, w[0], v);
+                    fma_bf8(v001, w[1], v);
+                    fma_bf8(v010, w[2], v);
+                    fma_bf8(v011, w[3], v);
+                    fma_bf8(v100, w[4], v);
+                    fma_bf8(v101, w[5], v);
+                    fma_bf8(v110, w[6], v);
+                    fma_bf8(v111, w[7], v);
+                    const float4 lo = make_float4(v[0], v[1], v[2], v[3]), hi = make_float4(v[4], v[5], v[6], v[7]);
+                    // with 8 lanes per row (64 channels) lanes 4..7 store their halves in the
+                    // other order, so each 8-lane phase of a store covers 32 distinct banks
+                    const bool swap = (gq & 4) != 0;
+                    st4(tile + j * kRow + 8 * gq + (swap ? 4 : 0), swap ? hi : lo);
+                    st4(tile + j * kRow + 8 * gq + (swap ? 0 : 4), swap ? lo : hi);
+                    if (to_slot) {
+                        const uint64_t pol = evict_last_policy();
+                        st4_keep(to_slot + j * kC + 8 * gq, lo, pol);
+                        st4_keep(to_slot + j * kC + 8 * gq + 4, hi, pol);
+                    }
+                } else {
+                    const float4 v000 = Store<S>::quad(p.data, e, ne), v001 = Store<S>::quad(p.data, e + kC, ne);
+                    const float4 v010 = Store<S>::quad(p.data, e + dy, ne),
+                                 v011 = Store<S>::quad(p.data, e + dy + kC, ne);
+                    const float4 v100 = Store<S>::quad(p.data, e + dz, ne),
+                                 v101 = Store<S>::quad(p.data, e + dz + kC, ne);
+                    const float4 v110 = Store<S>::quad(p.data, e + dz + dy, ne),
+                                 v111 = Store<S>::quad(p.data, e + dz + dy + kC, ne);
+                    float4 v = scale4(v000, w[0]);
+                    fma4(v, v001, w[1]);
+                    fma4(v, v010, w[2]);
+                    fma4(v, v011, w[3]);
+                    fma4(v, v100, w[4]);
+                    fma4(v, v101, w[5]);
+                    fma4(v, v110, w[6]);
+                    fma4(v, v111, w[7]);
+                    st4(tile + j * kRow + 4 * gq, v);
+                    if (to_slot) st4_keep(to_slot + j * kC + 4 * gq, v, evict_last_policy());
+                }
+            }
         }
-        st4(tile + j * kRow + 4 * q, v);
-        if (to_slot) st4_keep(to_slot + j * kC + 4 * q, v, evict_last_policy());
-    }
+        __syncwarp();
     }
     // one shading call site for both the gathered and the stashed rows (the kernel's code
-    // size sets how often its warps wait for instruction fetch)
-    __syncwarp();
-    if (s.shaded) {
-        // the row stays in shared memory; the shader reads the channels it needs from it
-        s.rgb = shade_any<kCompat, kDeg>(s.nrm, d, tile + lane * kRow, &s.spec);
-    } else {
-        s.rgb = f3{0.0f, 0.0f, 0.0f};
-        s.spec = f3{0.0f, 0.0f, 0.0f};
-    }
+    // size sets how often its warps wait for instruction fetch); the row stays in shared
+    // memory and the shader reads the channels it needs from it
+    if (s.shaded) s.rgb = shade_any<kCompat, kDeg>(s.nrm, d, tile + lane * kRow, &s.spec);
 }
 
 // Alpha only (no normal, gather or shading): what the backward-only pass needs to
 // rebuild the transmittance at each chunk start.  Validity matches eval_chunk.
 template <bool kCompat, typename S, int kVar>
 __device__ __forceinline__ void eval_alpha(const Params &p, uint32_t r, f3 o, f3 d, uint32_t nr, uint32_t chunk,
-                                           int lane, Sample &s) {
+                                           int lane, Sample &s, Edge &edge) {
     const uint32_t R = p.R;
     const uint32_t i = chunk * kWarp + lane;
     const bool live = i < nr;
-    bool ok = live;
     const float *tl = p.tlist ? QSDVR_AT(p.tlist, (uint64_t)kListT * r, kListT, (uint64_t)kListT * p.n) : nullptr;
     const CellPoint c1 = to_cell(tl ? at_t(o, d, live ? tl[i + 1] : 0.0f) : march(o, d, (float)(i + 1), p.interval),
                                  p.volume_offset, R);
     float s1 = 0.0f;
-    if (live) {
-        if (cell_in_grid(c1, R)) {
-            float a1[7];
-            load_cell<S, kVar>(p, c1, a1);
-            s1 = checked_sdf<kCompat>(a1, c1.u, (float)R);
-        } else {
-            ok = false;
-        }
+    uint32_t b1 = 0;
+    if (live && cell_in_grid(c1, R)) {
+        float a1[7];
+        load_cell<S, kVar>(p, c1, a1);
+        s1 = checked_sdf<kCompat>(a1, c1.u, (float)R);
+        b1 = edge_bits<kCompat>(s1);
     }
-    float s0 = __shfl_up_sync(kFull, s1, 1);
-    if (lane == 0 && live) {
-        const CellPoint c0 =
-            to_cell(tl ? at_t(o, d, tl[i]) : march(o, d, (float)i, p.interval), p.volume_offset, R);
-        if (cell_in_grid(c0, R)) {
-            float a0[7];
-            load_cell<S, kVar>(p, c0, a0);
-            s0 = checked_sdf<kCompat>(a0, c0.u, (float)R);
-        } else {
-            ok = false;
-        }
-    }
-    const bool ok_prev = __shfl_up_sync(kFull, ok, 1);
-    if (lane > 0) ok = ok && ok_prev;
-    if (live && !cell_in_grid(to_cell(tl ? at_t(o, d, 0.5f * (tl[i] + tl[i + 1])) : midpoint(o, d, i, p.interval),
-                                      p.volume_offset, R),
-                              R))
-        ok = false;
-    if (!kCompat && !(isfinite(s0) && isfinite(s1))) ok = false;
+    const uint32_t bits = chunk_terms<kCompat>(p, s1, b1, lane, edge, s.e0, s.e1);
+    const bool ok = live && bits == 3u &&
+                    cell_in_grid(to_cell(tl ? at_t(o, d, 0.5f * (tl[i] + tl[i + 1])) : midpoint(o, d, i, p.interval),
+                                         p.volume_offset, R),
+                                 R);
     s.valid = ok;
-    s.e0 = alpha_term<kCompat>(p.k, s0);
-    s.e1 = alpha_term<kCompat>(p.k, s1);
     s.alpha = ok ? interval_alpha<kCompat>(s.e0, s.e1) : 0.0f;
 }
 
@@ -709,14 +731,14 @@ __device__ __forceinline__ void corner_grads(float4 g, float px, float py, float
 }
 __device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 
-// Scatter the data-gradient tile (rows of 32 channels per lane's sample) through the
+// Scatter the data-gradient tile (a row per lane's sample, where it has one) through the
 // trilinear weights: 8 lanes per sample, one 16-byte RED (8 bytes for a bf16 gradient) per
 // lane and corner.  In the kVarMerge variant, samples of the chunk that lie in the same cell (same base
 // vertex) are found with one match_any: the first of them sums the others' weighted
 // contributions (their gradient rows and weights read from the tile) and sends one RED per
 // corner row for all of them; the others send nothing.
 template <int kDeg, int kVar>
-__device__ __forceinline__ void scatter_tile(const Params &p, float *tile, const Sample &s, int lane) {
+__device__ __forceinline__ void scatter_tile(const Params &p, float *tile, const Sample &s, bool has_row, int lane) {
     using RW = Rows<kDeg>;
     constexpr int kC = RW::kC, kRow = RW::kStride, kL = RW::kLanes, kPS = RW::kPerStep;
     const uint32_t R1 = p.R + 1, sy = R1, sz = R1 * R1;
@@ -725,14 +747,14 @@ __device__ __forceinline__ void scatter_tile(const Params &p, float *tile, const
     uint32_t others = 0;  // kVarMerge: the later samples of this lane's cell, summed into this one
     bool follower = false;
     if constexpr ((kVar & kVarMerge) != 0) {
-        const uint32_t key = s.valid ? s.vbase : (0x80000000u | (uint32_t)lane);  // vertices < 2^31
+        const uint32_t key = has_row ? s.vbase : (0x80000000u | (uint32_t)lane);  // vertices < 2^31
         const uint32_t peers = __match_any_sync(kFull, key);
         follower = (peers & ((1u << lane) - 1u)) != 0;  // a lower lane of the same cell leads
         others = follower ? 0u : (peers & ~(1u << lane));
     }
     // the row pad: (base vertex, or kNoVertex for a sample that sends nothing, and weights)
     st4(tile + lane * kRow + kC,
-        make_float4(__uint_as_float(s.valid && !follower ? s.vbase : kNoVertex), s.wx, s.wy, s.wz));
+        make_float4(__uint_as_float(has_row && !follower ? s.vbase : kNoVertex), s.wx, s.wy, s.wz));
     __syncwarp();
 // (one step per iteration: the REDs do not wait, and a smaller loop body keeps the kernel's
 // code small; measured as fast as two steps per iteration)
@@ -743,10 +765,10 @@ __device__ __forceinline__ void scatter_tile(const Params &p, float *tile, const
         const float4 w = ld4(tile + j * kRow + kC);
         const uint32_t vb = __float_as_uint(w.x);
         if (vb == kNoVertex) continue;
-        // A sample with alpha = 0 (the SDF does not fall across its interval) or T = 0 has a
-        // zero appearance gradient, as do channels its shader never reads: its 8 REDs would
-        // add zeros, yet each costs an L2 read-modify-write of a row that is usually not
-        // cached.  Skipped; the sums stay bit-identical (is_zero4).
+        // A sample with T = 0 has a zero appearance gradient, as do channels its shader never
+        // reads (one with alpha = 0 has no row at all): its 8 REDs would add zeros, yet each
+        // costs an L2 read-modify-write of a row that is usually not cached.  Skipped; the sums
+        // stay bit-identical (is_zero4).
         const float4 g = ld4(tile + j * kRow + 4 * q);
         if (is_zero4(g) && more == 0u) continue;
         float4 v[8];
@@ -842,6 +864,7 @@ __device__ __forceinline__ void backward_chunk(const Params &p, f3 o, f3 d, uint
     float from_next = __shfl_down_sync(kFull, mine_this, 1);
     if (lane == kWarp - 1) from_next = next_this;
     next_this = __shfl_sync(kFull, mine_this, 0);
+    bool has_row = false;  // this lane's row of the tile holds its data gradient
     if (s.valid) {
         // SDF sample i+1 and, for the ray's first lane, SDF sample 0
         const float gs1 = dl * d_next + (i + 1 < nr ? from_next : 0.0f);
@@ -853,7 +876,12 @@ __device__ __forceinline__ void backward_chunk(const Params &p, f3 o, f3 d, uint
         // every sample of the ray: then the unshaded one takes the full path too
         // (its zero row gives the same NaN outputs as the real row would)
         const f3 grgb{g.x * T * a, g.y * T * a, g.z * T * a};
-        if (s.shaded || !(isfinite(grgb.x) && isfinite(grgb.y) && isfinite(grgb.z))) {
+        has_row = s.shaded || !(isfinite(grgb.x) && isfinite(grgb.y) && isfinite(grgb.z));
+        if (has_row) {
+            if (!s.shaded) {
+#pragma unroll 1
+                for (int t = 0; t < kRow; t += 4) st4(tile + lane * kRow + t, make_float4(0.0f, 0.0f, 0.0f, 0.0f));
+            }
             // rgb gradient -> shader backward (data gradient into the tile, normal gradient)
             // data gradient written over the data row (every read precedes its write)
             const f3 gn =
@@ -871,8 +899,7 @@ __device__ __forceinline__ void backward_chunk(const Params &p, f3 o, f3 d, uint
                 scatter_cell<kVar>(p, s.cr, g7);
             }
         } else {
-            // alpha = 0: the colour's gradients (data row, normal) are 0 and the row
-            // in the tile is the gather's zeros, which the scatter skips
+            // alpha = 0: the colour's gradients (data row, normal) are 0; the sample has no row
             scatter_cell<kVar>(p, s.c1, gq);
         }
         if (i == 0) {
@@ -884,17 +911,42 @@ __device__ __forceinline__ void backward_chunk(const Params &p, f3 o, f3 d, uint
         }
     }
     __syncwarp();
-    scatter_tile<kDeg, kVar>(p, tile, s, lane);
+    scatter_tile<kDeg, kVar>(p, tile, s, has_row, lane);
     __syncwarp();
 }
 
+// The end of a persistent train pass: each warp adds its rays' squared errors (on lane 0) to one
+// of 32 partial sums and the last warp to finish adds those up, so that no sum is a chain of
+// thousands of additions in launch order (one float for all 2368 warps was off by 1e-6; 32 and
+// a tree by 1e-7).  Not inlined: inside the kernel it changed the main loop's register
+// allocation (bf16 degree 3 at 256^3: 2.44 instead of 2.20 ms).
+__device__ __noinline__ void finish_loss(uint32_t *counter, float *loss, float sq, uint32_t warp_id, uint32_t warps) {
+    const int lane = threadIdx.x & 31;
+    float *parts = reinterpret_cast<float *>(counter + kLossParts);
+    uint32_t done = 0;
+    if (lane == 0) {
+        atomicAdd(parts + warp_id % kWarp, sq);
+        asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(done) : "l"(counter + 1) : "memory");
+    }
+    if (__shfl_sync(kFull, done, 0) + 1 == warps) {
+        float v;
+        asm volatile("ld.acquire.gpu.global.f32 %0, [%1];" : "=f"(v) : "l"(parts + lane) : "memory");
+        const float sum = warp_sum(v);
+        if (lane == 0) atomicAdd(loss, sum);
+    }
+}
+
 template <bool kCompat, typename S, int kPass, bool kLogT, int kDeg, int kVar>
-__global__ void __launch_bounds__(kThreads, QSDVR_FUSED_MIN_BLOCKS) render_kernel(const Params p) {
+__global__ void __launch_bounds__(kThreads, min_blocks(kPass)) render_kernel(const Params p) {
     constexpr int kRow = Rows<kDeg>::kStride;
     constexpr uint32_t kChunkFloats = chunk_floats<kDeg>();
     __shared__ __align__(16) float tiles[kWarpsPerBlock][kWarp * kRow];
-    // the transmittance carry at each chunk start of the current ray, for the backward
-    __shared__ float carries[kWarpsPerBlock][kMaxChunks];
+    // the transmittance carry and the edge at each chunk start of the current ray, for the backward
+    // (a forward pass keeps none: shared memory it does not take is L1 for its gathers, and with
+    // 28 instead of 60 KB of L1 a 384^3 frame took 14 % longer)
+    constexpr uint32_t kCarries = kPass == kForward ? 1 : kMaxChunks;
+    __shared__ float carries[kWarpsPerBlock][kCarries], edge_es[kWarpsPerBlock][kCarries];
+    __shared__ uint8_t edge_bs[kWarpsPerBlock][kCarries];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     float *tile = tiles[w];
     const uint32_t warp_id = blockIdx.x * kWarpsPerBlock + w;
@@ -940,19 +992,27 @@ __global__ void __launch_bounds__(kThreads, QSDVR_FUSED_MIN_BLOCKS) render_kerne
         }
         Sample s;
         Transmittance<kLogT> tr;
-        float *carry_at = carries[w];  // carry_at[c]: the transmittance carry at the start of chunk c
+        // at the start of chunk c: the transmittance carry and the edge
+        float *carry_at = carries[w], *edge_e_at = edge_es[w];
+        uint8_t *edge_b_at = edge_bs[w];
+        Edge edge{0.0f, 0u};
+        if (run) edge = first_edge<kCompat, S, kVar>(p, r, o, d);
         float T_last = 0.0f;               // transmittance of this lane's sample in the last chunk
         // ---------------- forward (forward and backward-only passes)
         if (kPass == kForward || (kPass == kBackward && run)) {
             if (run) {
                 f3 acc{0.0f, 0.0f, 0.0f};
                 for (uint32_t c = 0; c < chunks; ++c) {
-                    if (lane == 0) carry_at[c] = tr.carry;  // warp-uniform
                     if (kPass == kBackward) {
-                        eval_alpha<kCompat, S, kVar>(p, r, o, d, nr, c, lane, s);
+                        if (lane == 0) {  // warp-uniform values
+                            carry_at[c] = tr.carry;
+                            edge_e_at[c] = edge.e;
+                            edge_b_at[c] = (uint8_t)edge.bits;
+                        }
+                        eval_alpha<kCompat, S, kVar>(p, r, o, d, nr, c, lane, s, edge);
                         tr.step(s.alpha, s.valid, lane);
                     } else {
-                        eval_chunk<kCompat, S, kDeg, kVar>(p, r, o, d, nr, c, lane, tile, s);
+                        eval_chunk<kCompat, S, kDeg, kVar>(p, r, o, d, nr, c, lane, tile, s, edge);
                         const float T = tr.step(s.alpha, s.valid, lane);
                         if (p.sample_alpha && c * kWarp + lane < nr) {
                             const uint64_t m = (uint64_t)info.render_offset + c * kWarp + lane;
@@ -976,7 +1036,8 @@ __global__ void __launch_bounds__(kThreads, QSDVR_FUSED_MIN_BLOCKS) render_kerne
             for (int c = (int)chunks - 1; c >= 0; --c) {
                 __syncwarp();
                 tr.carry = carry_at[c];
-                eval_chunk<kCompat, S, kDeg, kVar>(p, r, o, d, nr, (uint32_t)c, lane, tile, s);
+                edge = Edge{edge_e_at[c], edge_b_at[c]};
+                eval_chunk<kCompat, S, kDeg, kVar>(p, r, o, d, nr, (uint32_t)c, lane, tile, s, edge);
                 const float T = tr.step(s.alpha, s.valid, lane);
                 backward_chunk<kCompat, S, kDeg, kVar>(p, o, d, nr, (uint32_t)c, lane, tile, s, T, g, suf, next_this);
             }
@@ -1008,16 +1069,21 @@ __global__ void __launch_bounds__(kThreads, QSDVR_FUSED_MIN_BLOCKS) render_kerne
                 float T;
                 if (fwd || c + 1 < chunks) {
                     if (fwd) {
-                        if (lane == 0) carry_at[c] = tr.carry;  // warp-uniform
+                        if (lane == 0) {  // warp-uniform values
+                            carry_at[c] = tr.carry;
+                            edge_e_at[c] = edge.e;
+                            edge_b_at[c] = (uint8_t)edge.bits;
+                        }
                     } else {
                         __syncwarp();
                         tr.carry = carry_at[c];
+                        edge = Edge{edge_e_at[c], edge_b_at[c]};
                     }
                     float *sl = (slot && c + 1 < chunks && c + 1 + kSlotChunks >= chunks)
                                     ? slot + (c % kSlotChunks) * kChunkFloats
                                     : nullptr;
-                    eval_chunk<kCompat, S, kDeg, kVar>(p, r, o, d, nr, c, lane, tile, s, fwd ? nullptr : sl,
-                                                 fwd ? sl : nullptr);
+                    eval_chunk<kCompat, S, kDeg, kVar>(p, r, o, d, nr, c, lane, tile, s, edge,
+                                                       fwd ? nullptr : sl, fwd ? sl : nullptr);
                     T = tr.step(s.alpha, s.valid, lane);
                 } else {
                     // the forward just evaluated this chunk: its rows are still in the tile and
@@ -1043,7 +1109,13 @@ __global__ void __launch_bounds__(kThreads, QSDVR_FUSED_MIN_BLOCKS) render_kerne
     }
     if (!persistent) break;
     }  // ray loop
-    if (kPass == kTrain && lane == 0 && sq != 0.0f) atomicAdd(p.loss, sq);
+    if (kPass == kTrain) {
+        if (persistent) {
+            finish_loss(p.ray_counter, p.loss, sq, warp_id, gridDim.x * kWarpsPerBlock);
+        } else if (lane == 0 && sq != 0.0f) {
+            atomicAdd(p.loss, sq);
+        }
+    }
 }
 
 // ---- TMA brick staging for full frames (forward only, fixed mode, uniform march) --------
@@ -1238,6 +1310,7 @@ __global__ void __launch_bounds__(kBrickThreads) brick_frame_kernel(const __grid
 }
 
 constexpr size_t kCounterBytes = 256;
+static_assert((kLossParts + kWarp) * sizeof(uint32_t) <= kCounterBytes, "counters and partial sums share the area");
 
 // Calls f.template run<kCompat, S, kLogT, kDeg, kVar>() for the kernel configuration of `a`
 // (degree 3 exists only in the packed, fixed-mode layout; the separable SDF only with degree
@@ -1378,7 +1451,7 @@ int launch(const qsdvr_render_args *a, cudaStream_t stream) {
                              (unsigned long long)a->workspace_bytes, kPass == kTrain ? L.train_bytes : L.counter_bytes);
         p.ray_counter = static_cast<uint32_t *>(a->workspace);
         if (kPass == kTrain) p.slots = reinterpret_cast<float *>(static_cast<char *>(a->workspace) + kCounterBytes);
-        const int st = check_cuda(cudaMemsetAsync(p.ray_counter, 0, sizeof(uint32_t), stream), "render: memset");
+        const int st = check_cuda(cudaMemsetAsync(p.ray_counter, 0, kPass == kTrain ? kCounterBytes : sizeof(uint32_t), stream), "render: memset");
         if (st != QSDVR_OK) return st;
         blocks = L.blocks;
     }
