@@ -151,42 +151,137 @@ __device__ __forceinline__ bool adam_group(const AdamParams &a, uint64_t i, floa
     return true;
 }
 
+__device__ __forceinline__ void copy4(const AdamParams &a, uint64_t i, float4 p) {
+    __nv_bfloat162 lo = __floats2bfloat162_rn(p.x, p.y), hi = __floats2bfloat162_rn(p.z, p.w);
+    uint2 packed;
+    packed.x = *reinterpret_cast<uint32_t *>(&lo);
+    packed.y = *reinterpret_cast<uint32_t *>(&hi);
+    *reinterpret_cast<uint2 *>(a.copy + 4 * i) = packed;
+}
+
+// One element past the last whole group of 4.
+template <bool kBf16Grad>
+__device__ __forceinline__ void adam_tail(const AdamParams &a, uint64_t i) {
+    const float g = grad1<kBf16Grad>(a, i);
+    if (a.skip_zero && g == 0.0f) return;
+    __nv_bfloat16 *mb = reinterpret_cast<__nv_bfloat16 *>(a.m), *vb = reinterpret_cast<__nv_bfloat16 *>(a.v);
+    float p = a.param[i];
+    float m = a.state_bf16 ? __bfloat162float(mb[i]) : a.m[i], v = a.state_bf16 ? __bfloat162float(vb[i]) : a.v[i];
+    adam_one(p, g, m, v, a);
+    a.param[i] = p;
+    if (a.state_bf16) {
+        const uint32_t h = mix32(mix32((uint32_t)i ^ a.seed) ^ 0x51ed270bu);
+        mb[i] = __ushort_as_bfloat16((unsigned short)sr_bf16(m, h));
+        vb[i] = __ushort_as_bfloat16((unsigned short)sr_bf16(v, h >> 16));
+    } else {
+        a.m[i] = m;
+        a.v[i] = v;
+    }
+    if (a.zero_grad) {
+        if (kBf16Grad) reinterpret_cast<__nv_bfloat16 *>(a.grad)[i] = __float2bfloat16_rn(0.0f);
+        else a.grad[i] = 0.0f;
+    }
+    if (a.copy) a.copy[i] = __float2bfloat16_rn(p);
+}
+
+// Groups of 4 with a grid-stride loop: the lazy step (skip_zero), whose loads depend on the
+// gradient group by group, and buffers that are not 32-byte aligned.
 template <bool kBf16Grad>
 __global__ void __launch_bounds__(256) adam_kernel(const AdamParams a) {
     const uint64_t n4 = a.n / 4;
     const uint64_t stride = (uint64_t)gridDim.x * 256;
     for (uint64_t i = blockIdx.x * 256ull + threadIdx.x; i < n4; i += stride) {
         float4 p;
-        if (!adam_group<kBf16Grad>(a, i, p, false) || !a.copy) continue;
-        __nv_bfloat162 lo = __floats2bfloat162_rn(p.x, p.y), hi = __floats2bfloat162_rn(p.z, p.w);
-        uint2 packed;
-        packed.x = *reinterpret_cast<uint32_t *>(&lo);
-        packed.y = *reinterpret_cast<uint32_t *>(&hi);
-        *reinterpret_cast<uint2 *>(a.copy + 4 * i) = packed;
+        if (adam_group<kBf16Grad>(a, i, p, false) && a.copy) copy4(a, i, p);
     }
     // tail (n not a multiple of 4)
-    for (uint64_t i = 4 * n4 + blockIdx.x * 256ull + threadIdx.x; i < a.n; i += stride) {
-        const float g = grad1<kBf16Grad>(a, i);
-        if (a.skip_zero && g == 0.0f) continue;
-        __nv_bfloat16 *mb = reinterpret_cast<__nv_bfloat16 *>(a.m), *vb = reinterpret_cast<__nv_bfloat16 *>(a.v);
-        float p = a.param[i];
-        float m = a.state_bf16 ? __bfloat162float(mb[i]) : a.m[i], v = a.state_bf16 ? __bfloat162float(vb[i]) : a.v[i];
-        adam_one(p, g, m, v, a);
-        a.param[i] = p;
-        if (a.state_bf16) {
-            const uint32_t h = mix32(mix32((uint32_t)i ^ a.seed) ^ 0x51ed270bu);
-            mb[i] = __ushort_as_bfloat16((unsigned short)sr_bf16(m, h));
-            vb[i] = __ushort_as_bfloat16((unsigned short)sr_bf16(v, h >> 16));
-        } else {
-            a.m[i] = m;
-            a.v[i] = v;
+    for (uint64_t i = 4 * n4 + blockIdx.x * 256ull + threadIdx.x; i < a.n; i += stride) adam_tail<kBf16Grad>(a, i);
+}
+
+// The dense step, 8 elements a thread: 32-byte loads and stores (16-byte for bf16 streams), one
+// group per thread and as many blocks as that takes.  Bound by HBM: eight streams, of which a
+// warp touches 1 KB each.  With 16-byte accesses in a grid-stride loop of 16 blocks per SM the
+// streams' requests were too small and too few: the 671 M parameters of a 256^3 model (21.5 GB)
+// took 3.79 ms; with 32-byte accesses 3.36 ms, and 3.12 ms (6.88 TB/s) without the loop (blocks of
+// 512; 3.13 ms of 256).
+struct F8 {
+    float v[8];
+};
+__device__ __forceinline__ F8 ld8(const float *p) {
+    F8 r;
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(r.v[0]), "=f"(r.v[1]), "=f"(r.v[2]), "=f"(r.v[3]), "=f"(r.v[4]), "=f"(r.v[5]), "=f"(r.v[6]),
+                   "=f"(r.v[7])
+                 : "l"(p)
+                 : "memory");
+    return r;
+}
+__device__ __forceinline__ void st8(float *p, const F8 &r) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(r.v[0]), "f"(r.v[1]),
+                 "f"(r.v[2]), "f"(r.v[3]), "f"(r.v[4]), "f"(r.v[5]), "f"(r.v[6]), "f"(r.v[7])
+                 : "memory");
+}
+// 8 bf16 values as floats
+__device__ __forceinline__ F8 ld8_bf16(const float *base, uint64_t i) {
+    const uint4 r = reinterpret_cast<const uint4 *>(base)[i];
+    const float4 lo = bf16x4(make_uint2(r.x, r.y)), hi = bf16x4(make_uint2(r.z, r.w));
+    return F8{{lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w}};
+}
+__device__ __forceinline__ float4 half4(const F8 &r, int h) {
+    return make_float4(r.v[4 * h], r.v[4 * h + 1], r.v[4 * h + 2], r.v[4 * h + 3]);
+}
+
+constexpr int kDenseThreads = 512;
+template <bool kBf16Grad, bool kBf16State, bool kCells>
+__global__ void __launch_bounds__(kDenseThreads) adam_dense_kernel(const AdamParams a) {
+    const uint64_t i = blockIdx.x * (uint64_t)kDenseThreads + threadIdx.x;
+    if (i >= a.n / 8) return;
+    const F8 g = kBf16Grad ? ld8_bf16(a.grad, i) : ld8(a.grad + 8 * i);
+    F8 p = ld8(a.param + 8 * i);
+    F8 m = kBf16State ? ld8_bf16(a.m, i) : ld8(a.m + 8 * i), v = kBf16State ? ld8_bf16(a.v, i) : ld8(a.v + 8 * i);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) adam_one(p.v[q], g.v[q], m.v[q], v.v[q], a);
+    st8(a.param + 8 * i, p);
+    if (kBf16State) {
+        uint2 mr[2], vr[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {  // the random bits of group 2 i + h of 4, as adam_group draws them
+            const uint64_t j = 2 * i + h;
+            const uint32_t h0 = mix32((uint32_t)j ^ mix32((uint32_t)(j >> 32) ^ a.seed)), h1 = mix32(h0),
+                           h2 = mix32(h1), h3 = mix32(h2);
+            mr[h] = sr_bf16x4(half4(m, h), h0, h1);
+            vr[h] = sr_bf16x4(half4(v, h), h2, h3);
         }
-        if (a.zero_grad) {
-            if (kBf16Grad) reinterpret_cast<__nv_bfloat16 *>(a.grad)[i] = __float2bfloat16_rn(0.0f);
-            else a.grad[i] = 0.0f;
-        }
-        if (a.copy) a.copy[i] = __float2bfloat16_rn(p);
+        reinterpret_cast<uint4 *>(a.m)[i] = make_uint4(mr[0].x, mr[0].y, mr[1].x, mr[1].y);
+        reinterpret_cast<uint4 *>(a.v)[i] = make_uint4(vr[0].x, vr[0].y, vr[1].x, vr[1].y);
+    } else {
+        st8(a.m + 8 * i, m);
+        st8(a.v + 8 * i, v);
     }
+    if (a.zero_grad) {
+        if (kBf16Grad) reinterpret_cast<uint4 *>(a.grad)[i] = make_uint4(0u, 0u, 0u, 0u);
+        else st8(a.grad + 8 * i, F8{{0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f}});
+    }
+    if (a.copy) {
+        if (kCells) {  // the compensated cell form
+            reinterpret_cast<uint4 *>(a.copy)[i] = encode_sdf_cell(half4(p, 0), half4(p, 1));
+        } else {
+            copy4(a, 2 * i, half4(p, 0));
+            copy4(a, 2 * i + 1, half4(p, 1));
+        }
+    }
+}
+
+// What is left after the last whole group of 8: a group of 4, then single elements (one thread).
+template <bool kBf16Grad>
+__global__ void adam_rest_kernel(const AdamParams a) {
+    if (a.n & 4) {
+        const uint64_t i = a.n / 8 * 2;
+        float4 p;
+        adam_group<kBf16Grad>(a, i, p, false);
+        if (a.copy) copy4(a, i, p);
+    }
+    for (uint64_t e = a.n & ~3ull; e < a.n; ++e) adam_tail<kBf16Grad>(a, e);
 }
 
 // QSDVR_ADAM_SDF_CELLS: the parameters are quadric cells [n/8][8] with an fp32 gradient; one
@@ -251,16 +346,32 @@ extern "C" int qsdvr_adam_step(const qsdvr_adam_args *args, cudaStream_t stream)
     unsigned blocks = grid_for(work, 256);
     const unsigned cap = 148u * 16;  // a few waves of resident blocks, grid-stride beyond
     if (blocks > cap) blocks = cap;
-    if (args->flags & QSDVR_ADAM_SDF_CELLS) {
-        if (args->flags & QSDVR_ADAM_GRAD_BF16)
+    const bool cells = (args->flags & QSDVR_ADAM_SDF_CELLS) != 0, grad_bf16 = (args->flags & QSDVR_ADAM_GRAD_BF16) != 0;
+    // the dense kernel's accesses: 32 bytes of each fp32 stream, 16 of each bf16 one
+    const bool dense = !a.skip_zero && aligned(a.param, 32) && (grad_bf16 || aligned(a.grad, 32)) &&
+                       (a.state_bf16 || (aligned(a.m, 32) && aligned(a.v, 32)));
+    if (cells) {
+        if (grad_bf16)
             return set_error(QSDVR_ERR_INVALID_ARGUMENT, "qsdvr_adam_step: SDF cells take an fp32 gradient");
         if (args->count % 8 != 0 || (args->param_bf16 && !aligned(args->param_bf16, 16)))
             return set_error(QSDVR_ERR_INVALID_ARGUMENT,
                              "qsdvr_adam_step: SDF cells need a multiple of 8 elements and a 16-byte aligned copy");
+    }
+    if (dense) {
+        const unsigned n = grid_for(args->count / 8, kDenseThreads);
+        auto run = [&](auto kernel) { kernel<<<n, kDenseThreads, 0, stream>>>(a); };
+        if (cells) a.state_bf16 ? run(adam_dense_kernel<false, true, true>) : run(adam_dense_kernel<false, false, true>);
+        else if (grad_bf16) a.state_bf16 ? run(adam_dense_kernel<true, true, false>) : run(adam_dense_kernel<true, false, false>);
+        else a.state_bf16 ? run(adam_dense_kernel<false, true, false>) : run(adam_dense_kernel<false, false, false>);
+        if (args->count % 8) {
+            if (grad_bf16) adam_rest_kernel<true><<<1, 1, 0, stream>>>(a);
+            else adam_rest_kernel<false><<<1, 1, 0, stream>>>(a);
+        }
+    } else if (cells) {
         unsigned cblocks = grid_for(args->count / 8, 256);
         if (cblocks > cap) cblocks = cap;
         adam_cells_kernel<<<cblocks, 256, 0, stream>>>(a);
-    } else if (args->flags & QSDVR_ADAM_GRAD_BF16) {
+    } else if (grad_bf16) {
         adam_kernel<true><<<blocks, 256, 0, stream>>>(a);
     } else {
         adam_kernel<false><<<blocks, 256, 0, stream>>>(a);
