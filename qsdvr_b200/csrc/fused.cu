@@ -6,8 +6,8 @@
 // Work mapping (one warp per ray, 32 render samples per "chunk"):
 //   * lane i owns render sample i of the chunk: its positions (bit-exact with
 //     GenerateRayPoints), quadric cells, SDF values, normal, alpha and shading;
-//   * the 32-channel appearance rows are gathered with 16-byte loads by groups of 8 lanes
-//     (one float4 each) or 4 lanes (bf16 x 8 each), so every load covers whole 128-byte
+//   * the 32-channel appearance rows are gathered with 32-byte loads by groups of 4 lanes
+//     (8 floats each) or 2 lanes (16 bf16 each), so every load covers whole 128-byte
 //     (64-byte bf16) vertex rows, interpolated and staged in a per-warp shared-memory
 //     tile [32][36] floats
 //     (row stride 36 keeps both the row-wise and the lane-wise float4 accesses
@@ -46,7 +46,7 @@ namespace {
 #define QSDVR_FORWARD_MIN_BLOCKS 20
 #endif
 #ifndef QSDVR_GATHER_UNROLL
-#define QSDVR_GATHER_UNROLL 2
+#define QSDVR_GATHER_UNROLL 1
 #endif
 constexpr int kWarpsPerBlock = QSDVR_FUSED_WARPS;
 constexpr int kGatherUnroll = QSDVR_GATHER_UNROLL;
@@ -146,6 +146,7 @@ struct Params {
     uint64_t sample_capacity;
     const uint32_t *order;  // optional: the i-th ray taken is order[i]
     bool grad_bf16;         // data_grad holds bf16 values
+    bool wide;              // data is 32-byte aligned: the gather's loads are 32 bytes a lane
 };
 
 constexpr uint32_t kListT = 33;  // list sampling: 33 SDF positions, 32 render samples per ray
@@ -176,10 +177,6 @@ struct Store<float> {
         a[0] = lo.x; a[1] = lo.y; a[2] = lo.z; a[3] = lo.w;
         a[4] = hi.x; a[5] = hi.y; a[6] = hi.z;
     }
-    // elements [e, e + 4) of the appearance grid: one 16-byte load
-    __device__ static float4 quad(const void *d, uint64_t e, [[maybe_unused]] uint64_t extent) {
-        return ld4(QSDVR_AT(static_cast<const float *>(d), e, 4, extent));
-    }
 };
 
 template <>
@@ -192,23 +189,35 @@ struct Store<__nv_bfloat16> {
         // into two bf16; exact in fp32)
         a[4] = bf_lo(r.z); a[5] = bf_hi(r.z); a[6] = bf_lo(r.w) + bf_hi(r.w);
     }
-    // elements [e, e + 8) of the appearance grid: one 16-byte load (bf16 x 8)
-    __device__ static uint4 oct(const void *d, uint64_t e, [[maybe_unused]] uint64_t extent) {
-        return *reinterpret_cast<const uint4 *>(QSDVR_AT(static_cast<const __nv_bfloat16 *>(d), e, 8, extent));
-    }
 };
 
-// Lanes of the appearance gather: each lane loads 16 bytes of a vertex row per corner (a
-// float4 of fp32 storage, 8 x bf16 of bf16 storage), so kLanes lanes cover one row and a warp
-// instruction fetches kPerStep samples' rows.
+// Lanes of the appearance gather: each lane takes 32 bytes of a vertex row per corner (8 fp32 or
+// 16 bf16 channels), so kLanes lanes cover one row and a warp instruction fetches kPerStep
+// samples' rows.  32-byte loads halve the gather's instructions per byte (loads, addresses,
+// weights), which the issue-bound frames feel: 384^3 frame 5.92 -> 5.36 ms, its proposal form
+// 1.79 -> 1.70 ms, fp32 degree 3 at 128^3 (autograd) 0.427 -> 0.407 ms; the fp32 degree-2 training
+// batches, which memory bounds, stay as they were.
 template <typename S, int kDeg>
 struct GatherLanes {
     static constexpr int kC = ShLayout<kDeg>::kChannels;
-    static constexpr int kCh = 16 / (int)sizeof(S);  // channels per lane
+    static constexpr int kCh = 32 / (int)sizeof(S);  // channels per lane
     static constexpr int kLanes = kC / kCh;
     static constexpr int kPerStep = kWarp / kLanes;
 };
 
+// 32 bytes at p: one load where the grid is 32-byte aligned, else two.
+template <bool kWide>
+__device__ __forceinline__ void ld32(const void *p, uint32_t (&r)[8]) {
+    if (kWide) {
+        asm("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+            : "l"(p));
+    } else {
+        const uint4 lo = static_cast<const uint4 *>(p)[0], hi = static_cast<const uint4 *>(p)[1];
+        r[0] = lo.x; r[1] = lo.y; r[2] = lo.z; r[3] = lo.w;
+        r[4] = hi.x; r[5] = hi.y; r[6] = hi.z; r[7] = hi.w;
+    }
+}
 
 __device__ __forceinline__ void red_cell(float *g8, uint32_t cell, const float *g, uint64_t cells) {
     float *b = QSDVR_AT(g8, 8ull * cell, 8, 8 * cells);
@@ -247,6 +256,7 @@ __device__ __forceinline__ void sep_red(float4 *sg, uint32_t R, const CellPoint 
 // kernel's code size sets how often its warps wait for instruction fetch).
 constexpr int kVarSep = 1;    // separable SDF tables instead of the dense cell grid
 constexpr int kVarMerge = 2;  // same-cell merged appearance scatter
+constexpr int kVarNarrow = 4; // the plain kernel for an appearance grid that is not 32-byte aligned
 
 template <typename S, int kVar>
 __device__ __forceinline__ void load_cell(const Params &p, const CellPoint &c, float *a) {
@@ -306,6 +316,24 @@ __device__ __forceinline__ void fma_bf8(uint4 r, float w, float *v) {
     const uint32_t rv[4] = {r.x, r.y, r.z, r.w};
 #pragma unroll
     for (int t = 0; t < 4; ++t) ffma2(v[2 * t], v[2 * t + 1], w, bf_lo(rv[t]), bf_hi(rv[t]));
+}
+
+// v = w * (the channels of 32 bytes r), or v += w * (...)
+template <typename S, bool kFirst>
+__device__ __forceinline__ void weigh32(const uint32_t (&r)[8], float w, float *v) {
+#pragma unroll
+    for (int t = 0; t < 8; t += sizeof(S) == 2 ? 1 : 2) {
+        // the next two channels: a pair of bf16 or two floats
+        const float x0 = sizeof(S) == 2 ? bf_lo(r[t]) : __uint_as_float(r[t]);
+        const float x1 = sizeof(S) == 2 ? bf_hi(r[t]) : __uint_as_float(r[(t + 1) & 7]);
+        float *o = v + (sizeof(S) == 2 ? 2 * t : t);
+        if (kFirst) {
+            o[0] = w * x0;
+            o[1] = w * x1;
+        } else {
+            ffma2(o[0], o[1], w, x0, x1);
+        }
+    }
 }
 
 __device__ __forceinline__ float warp_sum(float v) {
@@ -460,6 +488,56 @@ __device__ __forceinline__ uint32_t chunk_terms(const Params &p, float s1, uint3
     return b0 & b1;
 }
 
+// The interpolated rows of a chunk's shaded samples into the tile (and, if to_slot, the stash).
+// Groups of GatherLanes::kLanes lanes fetch one sample's 8 corner rows, kPerStep samples per step;
+// samples without a colour are skipped.
+template <typename S, int kDeg, bool kWide>
+__device__ __forceinline__ void gather_rows(const Params &p, float *tile, uint32_t shaded, int lane, float *to_slot) {
+    using GL = GatherLanes<S, kDeg>;
+    constexpr int kC = GL::kC, kRow = Rows<kDeg>::kStride, kGL = GL::kLanes, kGPS = GL::kPerStep, kCh = GL::kCh;
+    constexpr int kRound = kGPS * kGatherUnroll;
+    constexpr uint32_t kRoundMask = kRound >= 32 ? 0xffffffffu : (1u << (kRound & 31)) - 1u;
+    const uint32_t R1 = p.R + 1;
+    const uint64_t dy = (uint64_t)kC * R1, dz = dy * R1;  // elements to the rows above in y and z
+    [[maybe_unused]] const uint64_t ne = dz * R1;
+    const int gq = lane % kGL;
+#pragma unroll 1
+    for (int first = 0; first < kWarp; first += kRound) {
+        if (((shaded >> first) & kRoundMask) == 0) continue;  // warp-uniform
+#pragma unroll
+        for (int u = 0; u < kGatherUnroll; ++u) {
+            const int j = first + u * kGPS + lane / kGL;
+            const float4 prm = ld4(tile + j * kRow + kC);
+            const uint32_t vb = __float_as_uint(prm.x);
+            if (vb == kNoVertex) continue;
+            const uint64_t e = (uint64_t)kC * vb + kCh * gq;
+            const S *d = static_cast<const S *>(p.data);
+            float w[8], v[kCh];
+            corner_weights(prm.y, prm.z, prm.w, w);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {  // the corners of the lower and of the upper z plane
+                const uint64_t ez = h ? e + dz : e;
+                uint32_t r[4][8];
+                ld32<kWide>(QSDVR_AT(d, ez, kCh, ne), r[0]);
+                ld32<kWide>(QSDVR_AT(d, ez + kC, kCh, ne), r[1]);
+                ld32<kWide>(QSDVR_AT(d, ez + dy, kCh, ne), r[2]);
+                ld32<kWide>(QSDVR_AT(d, ez + dy + kC, kCh, ne), r[3]);
+                if (h == 0) weigh32<S, true>(r[0], w[0], v);
+                else weigh32<S, false>(r[0], w[4], v);
+                weigh32<S, false>(r[1], w[4 * h + 1], v);
+                weigh32<S, false>(r[2], w[4 * h + 2], v);
+                weigh32<S, false>(r[3], w[4 * h + 3], v);
+            }
+#pragma unroll
+            for (int t = 0; t < kCh; t += 4) {
+                const float4 q = make_float4(v[t], v[t + 1], v[t + 2], v[t + 3]);
+                st4(tile + j * kRow + kCh * gq + t, q);
+                if (to_slot) st4_keep(to_slot + j * kC + kCh * gq + t, q, evict_last_policy());
+            }
+        }
+    }
+}
+
 // Forward evaluation of render sample i = chunk*32 + lane (kernel/camera.cu:60-96,
 // kernel/surface.cu:54-115, kernel/render.cu:98-179, :239-244).  Leaves the interpolated
 // channels of the shaded samples in their rows of the warp's tile (the other rows are not
@@ -532,7 +610,7 @@ __device__ __forceinline__ void eval_chunk(const Params &p, uint32_t r, f3 o, f3
 #if QSDVR_GATHER_PREFETCH
     if constexpr (QSDVR_GATHER_PREFETCH == 2 || kDeg == 2) {
         // samples of the gather's first round of loads (issued right below) are not prefetched
-        constexpr int kRound = (sizeof(S) == 2 ? GatherLanes<S, kDeg>::kPerStep : kPS) * kGatherUnroll;
+        constexpr int kRound = GatherLanes<S, kDeg>::kPerStep * kGatherUnroll;
         if (!from_slot && s.shaded && lane >= kRound) {
             constexpr uint32_t kPair = 2u * kC * sizeof(S);  // rows v and v + 1 are adjacent
             const S *base = static_cast<const S *>(p.data);
@@ -568,73 +646,15 @@ __device__ __forceinline__ void eval_chunk(const Params &p, uint32_t r, f3 o, f3
     } else {
         st4(tile + lane * kRow + kC, make_float4(__uint_as_float(s.shaded ? s.vbase : kNoVertex), s.wx, s.wy, s.wz));
         __syncwarp();
-        // Groups of kGL lanes fetch one sample's 8 corner rows (16 bytes a lane and corner), kGPS
-        // samples per step, kGatherUnroll steps at a time; samples without a colour are skipped.
-        using GL = GatherLanes<S, kDeg>;
-        constexpr int kGL = GL::kLanes, kGPS = GL::kPerStep, kCh = GL::kCh, kRound = kGPS * kGatherUnroll;
-        constexpr uint32_t kRoundMask = kRound >= 32 ? 0xffffffffu : (1u << (kRound & 31)) - 1u;
-        const uint64_t dy = (uint64_t)kC * sy, dz = (uint64_t)kC * sz, ne = nv * kC;  // in elements
-        const int gq = lane % kGL;
-#pragma unroll 1
-        for (int first = 0; first < kWarp; first += kRound) {
-            if (((shaded >> first) & kRoundMask) == 0) continue;  // warp-uniform
-#pragma unroll
-            for (int u = 0; u < kGatherUnroll; ++u) {
-                const int j = first + u * kGPS + lane / kGL;
-                const float4 prm = ld4(tile + j * kRow + kC);
-                const uint32_t vb = __float_as_uint(prm.x);
-                if (vb == kNoVertex) continue;
-                const uint64_t e = (uint64_t)kC * vb + kCh * gq;
-                float w[8];
-                corner_weights(prm.y, prm.z, prm.w, w);
-                if constexpr (sizeof(S) == 2) {
-                    const uint4 v000 = Store<S>::oct(p.data, e, ne), v001 = Store<S>::oct(p.data, e + kC, ne);
-                    const uint4 v010 = Store<S>::oct(p.data, e + dy, ne),
-                                v011 = Store<S>::oct(p.data, e + dy + kC, ne);
-                    const uint4 v100 = Store<S>::oct(p.data, e + dz, ne),
-                                v101 = Store<S>::oct(p.data, e + dz + kC, ne);
-                    const uint4 v110 = Store<S>::oct(p.data, e + dz + dy, ne),
-                                v111 = Store<S>::oct(p.data, e + dz + dy + kC, ne);
-                    float v[8];
-                    first_bf8(v000, w[0], v);
-                    fma_bf8(v001, w[1], v);
-                    fma_bf8(v010, w[2], v);
-                    fma_bf8(v011, w[3], v);
-                    fma_bf8(v100, w[4], v);
-                    fma_bf8(v101, w[5], v);
-                    fma_bf8(v110, w[6], v);
-                    fma_bf8(v111, w[7], v);
-                    const float4 lo = make_float4(v[0], v[1], v[2], v[3]), hi = make_float4(v[4], v[5], v[6], v[7]);
-                    // with 8 lanes per row (64 channels) lanes 4..7 store their halves in the
-                    // other order, so each 8-lane phase of a store covers 32 distinct banks
-                    const bool swap = (gq & 4) != 0;
-                    st4(tile + j * kRow + 8 * gq + (swap ? 4 : 0), swap ? hi : lo);
-                    st4(tile + j * kRow + 8 * gq + (swap ? 0 : 4), swap ? lo : hi);
-                    if (to_slot) {
-                        const uint64_t pol = evict_last_policy();
-                        st4_keep(to_slot + j * kC + 8 * gq, lo, pol);
-                        st4_keep(to_slot + j * kC + 8 * gq + 4, hi, pol);
-                    }
-                } else {
-                    const float4 v000 = Store<S>::quad(p.data, e, ne), v001 = Store<S>::quad(p.data, e + kC, ne);
-                    const float4 v010 = Store<S>::quad(p.data, e + dy, ne),
-                                 v011 = Store<S>::quad(p.data, e + dy + kC, ne);
-                    const float4 v100 = Store<S>::quad(p.data, e + dz, ne),
-                                 v101 = Store<S>::quad(p.data, e + dz + kC, ne);
-                    const float4 v110 = Store<S>::quad(p.data, e + dz + dy, ne),
-                                 v111 = Store<S>::quad(p.data, e + dz + dy + kC, ne);
-                    float4 v = scale4(v000, w[0]);
-                    fma4(v, v001, w[1]);
-                    fma4(v, v010, w[2]);
-                    fma4(v, v011, w[3]);
-                    fma4(v, v100, w[4]);
-                    fma4(v, v101, w[5]);
-                    fma4(v, v110, w[6]);
-                    fma4(v, v111, w[7]);
-                    st4(tile + j * kRow + 4 * gq, v);
-                    if (to_slot) st4_keep(to_slot + j * kC + 4 * gq, v, evict_last_policy());
-                }
-            }
+        // (both forms in one kernel cost the plain one 1 %, so its narrow form is an instance of
+        // its own; the separable and the merged kernels choose at run time)
+        if constexpr (kVar == 0) {
+            gather_rows<S, kDeg, true>(p, tile, shaded, lane, to_slot);
+        } else if constexpr (kVar == kVarNarrow) {
+            gather_rows<S, kDeg, false>(p, tile, shaded, lane, to_slot);
+        } else {
+            if (p.wide) gather_rows<S, kDeg, true>(p, tile, shaded, lane, to_slot);
+            else gather_rows<S, kDeg, false>(p, tile, shaded, lane, to_slot);
         }
         __syncwarp();
     }
@@ -1321,6 +1341,8 @@ void with_variant(const qsdvr_render_args *a, F &f) {
         if constexpr (D == 2) f.template run<C, S, L, D, kVarSep>();
     } else if (a->merge_scatter) {
         f.template run<C, S, L, D, kVarMerge>();
+    } else if (!aligned(a->data, 32)) {
+        f.template run<C, S, L, D, kVarNarrow>();
     } else {
         f.template run<C, S, L, D, 0>();
     }
@@ -1345,7 +1367,8 @@ void dispatch(const qsdvr_render_args *a, F &f) {
     }
 }
 
-// The forward pass scatters nothing: its merged variant is the plain one.
+// The forward pass scatters nothing: it has no merged instance (launch and layout_for clear the
+// option for it, so that an unaligned grid finds its way to kVarNarrow).
 template <int kPass, int kVar>
 constexpr int pass_variant() { return kPass == kForward ? (kVar & ~kVarMerge) : kVar; }
 
@@ -1390,7 +1413,12 @@ Layout layout_for(const qsdvr_render_args *a, int pass = kTrain) {
     }
     Occupancy occ;
     occ.pass = pass;
-    dispatch(a, occ);
+    // the grid and the workspace do not depend on the grid's alignment: a size that was asked for
+    // before the pointers were known stays right
+    qsdvr_render_args variant = *a;
+    variant.data = nullptr;
+    if (pass == kForward) variant.merge_scatter = 0;
+    dispatch(&variant, occ);
     if (check_cuda(occ.err, "render: occupancy") != QSDVR_OK) {
         L.error = QSDVR_ERR_CUDA;
         return L;
@@ -1442,6 +1470,7 @@ int launch(const qsdvr_render_args *a, cudaStream_t stream) {
     p.sample_capacity = a->sample_capacity;
     p.order = a->order;
     p.grad_bf16 = a->data_grad_storage == QSDVR_STORAGE_BF16;
+    p.wide = aligned(a->data, 32);
     unsigned blocks = grid_for(a->ray_count, kWarpsPerBlock);
     if (a->workspace) {
         const Layout L = layout_for(a, kPass);
@@ -1456,7 +1485,9 @@ int launch(const qsdvr_render_args *a, cudaStream_t stream) {
         blocks = L.blocks;
     }
     Launcher<kPass> launcher{&p, blocks, stream};
-    dispatch(a, launcher);
+    qsdvr_render_args variant = *a;
+    if (kPass == kForward) variant.merge_scatter = 0;
+    dispatch(&variant, launcher);
     return check_launch(kPass == kForward ? "qsdvr_render_forward"
                                           : (kPass == kBackward ? "qsdvr_render_backward" : "qsdvr_render_train"));
 }
