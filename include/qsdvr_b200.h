@@ -299,7 +299,7 @@ int qsdvr_ray_order_keys(const qsdvr_ray_info *rays, const float *origin, const 
                          float interval, uint32_t *keys, cudaStream_t stream);
 
 /* Workspace bytes of qsdvr_ray_order for ray_count rays (a 2^15 + 1 bucket histogram and one
- * bucket per ray). */
+ * rank per ray). */
 size_t qsdvr_ray_order_workspace_size(uint32_t ray_count);
 
 /* The ray order itself, without a library sort (no counterpart in the reference): order

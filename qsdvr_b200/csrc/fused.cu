@@ -1571,8 +1571,8 @@ __global__ void __launch_bounds__(256) ray_order_keys_kernel(const qsdvr_ray_inf
 
 // Ray order by counting sort: the 15-bit Morton code of each ray's in-box midpoint (5 bits
 // per axis, a 32^3 lattice of the volume; rays without samples in one extra last bucket),
-// a histogram, its exclusive scan, and a scatter that lists each bucket's rays in the order
-// the scatter reaches them.  Rays in one bucket lie within one 1/16-wide cube of the volume,
+// a histogram that also ranks each bucket's rays in the order its atomics reach them, its
+// exclusive scan, and a scatter.  Rays in one bucket lie within one 1/16-wide cube of the volume,
 // the locality the render kernels need; finer keys order rays within such a cube, which does
 // not change what the rays in flight share.
 constexpr uint32_t kOrderBuckets = (1u << 15) + 1;
@@ -1594,16 +1594,30 @@ __device__ __forceinline__ uint32_t ray_bucket(const qsdvr_ray_info *rays, const
     return spread3(q[0]) | (spread3(q[1]) << 1) | (spread3(q[2]) << 2);
 }
 
-__global__ void __launch_bounds__(256) ray_bucket_kernel(const qsdvr_ray_info *__restrict__ rays,
-                                                         const float *__restrict__ origin,
-                                                         const float *__restrict__ dir, uint32_t n, float interval,
-                                                         const float *__restrict__ tlist, uint32_t *__restrict__ bucket,
-                                                         uint32_t *__restrict__ hist) {
+// The histogram, and each ray's rank among the rays that reached its bucket before it.  The rays
+// without samples (a quarter of a batch of views) share one bucket: a warp counts its own with one
+// atomic, since one per ray queued up on that counter and was most of this kernel's time, and of
+// the scatter's, which took another atomic per ray where the rank serves now (it finds the bucket
+// again from the ray): 65536 rays 11.6 + 11.5 -> 4.4 + 2.8 us.
+__global__ void __launch_bounds__(256) ray_rank_kernel(const qsdvr_ray_info *__restrict__ rays,
+                                                       const float *__restrict__ origin,
+                                                       const float *__restrict__ dir, uint32_t n, float interval,
+                                                       const float *__restrict__ tlist, uint32_t *__restrict__ rank,
+                                                       uint32_t *__restrict__ hist) {
     const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= n) return;
-    const uint32_t b = ray_bucket(rays, origin, dir, r, n, interval, tlist);
-    bucket[r] = b;
-    atomicAdd(hist + b, 1u);
+    const uint32_t b = r < n ? ray_bucket(rays, origin, dir, r, n, interval, tlist) : 0u;
+    const bool empty = r < n && b == kOrderBuckets - 1;
+    const uint32_t peers = __ballot_sync(kFull, empty), lane = threadIdx.x & 31;
+    uint32_t k = 0;
+    if (r < n && !empty) k = atomicAdd(hist + b, 1u);
+    if (peers) {
+        const int leader = __ffs(peers) - 1;
+        uint32_t base = 0;
+        if ((int)lane == leader) base = atomicAdd(hist + (kOrderBuckets - 1), (uint32_t)__popc(peers));
+        base = __shfl_sync(kFull, base, leader);
+        if (empty) k = base + __popc(peers & ((1u << lane) - 1u));
+    }
+    if (r < n) rank[r] = k;
 }
 
 // Exclusive scan of the kOrderBuckets counts in place, one block of 1024 threads.  Each
@@ -1663,11 +1677,16 @@ __global__ void __launch_bounds__(1024) bucket_scan_kernel(uint32_t *__restrict_
     }
 }
 
-__global__ void __launch_bounds__(256) ray_scatter_kernel(const uint32_t *__restrict__ bucket, uint32_t n,
-                                                          uint32_t *__restrict__ next, uint32_t *__restrict__ order) {
+__global__ void __launch_bounds__(256) ray_scatter_kernel(const qsdvr_ray_info *__restrict__ rays,
+                                                          const float *__restrict__ origin,
+                                                          const float *__restrict__ dir, uint32_t n, float interval,
+                                                          const float *__restrict__ tlist,
+                                                          const uint32_t *__restrict__ rank,
+                                                          const uint32_t *__restrict__ first,
+                                                          uint32_t *__restrict__ order) {
     const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= n) return;
-    const uint32_t pos = atomicAdd(next + bucket[r], 1u);
+    const uint32_t pos = first[ray_bucket(rays, origin, dir, r, n, interval, tlist)] + rank[r];
     if (pos < n) order[pos] = r;
     else flag_error(QSDVR_DEVERR_CAPACITY);
 }
@@ -1713,7 +1732,7 @@ int ray_order(const char *fn, const qsdvr_ray_info *rays, const float *origin, c
     if (!workspace || workspace_bytes < need || !aligned(workspace, 4))
         return set_error(QSDVR_ERR_WORKSPACE, "%s: workspace %zu < %zu bytes (4-byte aligned)", fn, workspace_bytes,
                          need);
-    uint32_t *hist = static_cast<uint32_t *>(workspace), *bucket = hist + kOrderBuckets;
+    uint32_t *hist = static_cast<uint32_t *>(workspace), *rank = hist + kOrderBuckets;
     const int st = check_cuda(cudaMemsetAsync(hist, 0, kOrderBuckets * sizeof(uint32_t), stream), fn);
     if (st != QSDVR_OK) return st;
     // (the scan's shared memory is above the default 48 KB; the attribute is set on the
@@ -1722,9 +1741,9 @@ int ray_order(const char *fn, const qsdvr_ray_info *rays, const float *origin, c
         cudaFuncSetAttribute(bucket_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kScanSmem), fn);
     if (sa != QSDVR_OK) return sa;
     const unsigned blocks = grid_for(ray_count, 256);
-    ray_bucket_kernel<<<blocks, 256, 0, stream>>>(rays, origin, dir, ray_count, interval, tlist, bucket, hist);
+    ray_rank_kernel<<<blocks, 256, 0, stream>>>(rays, origin, dir, ray_count, interval, tlist, rank, hist);
     bucket_scan_kernel<<<1, 1024, kScanSmem, stream>>>(hist);
-    ray_scatter_kernel<<<blocks, 256, 0, stream>>>(bucket, ray_count, hist, order);
+    ray_scatter_kernel<<<blocks, 256, 0, stream>>>(rays, origin, dir, ray_count, interval, tlist, rank, hist, order);
     return check_launch(fn);
 }
 }  // namespace
