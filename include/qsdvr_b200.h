@@ -333,8 +333,10 @@ int qsdvr_separable_sdf_grad(float *table_grad, uint32_t reso, float *x_grad, fl
                              float *offset_grad, cudaStream_t stream);
 
 /* Workspace bytes for qsdvr_render_* with these args on the current device (mode, storage
- * and transmittance select the kernel; independent of ray_count).  One workspace must not
- * be used by launches that may overlap on the GPU. */
+ * and transmittance select the kernel; independent of ray_count; with sdf_layers it holds the
+ * copies of the table gradient that the train and backward passes add to, 64 x (3 reso + 1) x 16
+ * bytes: a smaller workspace works without them).  One workspace must not be used by launches
+ * that may overlap on the GPU. */
 size_t qsdvr_render_workspace_size(const qsdvr_render_args *args);
 
 /* Replaces RenderGrid.forward (models/render.py:225-234, i.e. the SampleSDF, SampleNormal,

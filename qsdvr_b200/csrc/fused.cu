@@ -141,6 +141,7 @@ struct Params {
     uint32_t *ray_counter;  // persistent mode: next ray to take (zeroed before the launch), then
                             // in train mode the warps that are done and the loss's partial sums
     float *slots;           // persistent train mode: per-warp row stash, kSlotChunks chunks each
+    float4 *sep_copies;     // separable gradient: kSepCopies tables that the warps share out, or null
     const float *tlist;     // list sampling: per ray kListT SDF positions (t from origin), or null
     float *sample_alpha;    // optional per-render-sample alpha output (forward, train)
     uint64_t sample_capacity;
@@ -243,6 +244,14 @@ __device__ __forceinline__ void sep_cell(const float4 *sep, uint32_t R, const Ce
 
 // Its adjoint: one 16-byte RED per axis row.  The off3 gradient (the sum of every cell's g6)
 // is recovered from the x rows' g6 sums by the reverse recurrence, so it needs no atomics.
+// Every sample of a batch adds to the same 3R rows, and their L2 lines' turns at the atomics were
+// what bound the pass; with a workspace the warps add to one of kSepCopies tables there, which
+// sep_sum_kernel sums into the caller's: 65536 rays at 64^3 1.41 -> 0.88 ms, at 256^3 1.94 ->
+// 1.73 ms (16 copies the same, 256 1.76 ms).
+#ifndef QSDVR_SEP_COPIES
+#define QSDVR_SEP_COPIES 64
+#endif
+constexpr uint32_t kSepCopies = QSDVR_SEP_COPIES;
 __device__ __forceinline__ void sep_red(float4 *sg, uint32_t R, const CellPoint &c, const float *g) {
     [[maybe_unused]] const uint64_t n = 3ull * R + 1;
     const float4 x = make_float4(g[0], g[3], g[6], 0.0f), y = make_float4(g[1], g[4], g[6], 0.0f),
@@ -266,7 +275,8 @@ __device__ __forceinline__ void load_cell(const Params &p, const CellPoint &c, f
 
 template <int kVar>
 __device__ __forceinline__ void scatter_cell(const Params &p, const CellPoint &c, const float *g) {
-    if constexpr ((kVar & kVarSep) != 0) sep_red(p.sep_grad, p.R, c, g);
+    if constexpr ((kVar & kVarSep) != 0)
+        sep_red(p.sep_copies ? p.sep_copies + (uint64_t)(blockIdx.x % kSepCopies) * (3 * p.R + 1) : p.sep_grad, p.R, c, g);
     else red_cell(p.sdf_grad, (uint32_t)c.index, g, (uint64_t)p.R * p.R * p.R);
 }
 
@@ -1329,6 +1339,22 @@ __global__ void __launch_bounds__(kBrickThreads) brick_frame_kernel(const __grid
     if (r < p.n) store3(QSDVR_AT(p.color, 3ull * r, 3, 3ull * p.n), acc);
 }
 
+// grad[i] += the sum of the copies' entries i, a warp per table row.
+__global__ void __launch_bounds__(256) sep_sum_kernel(const float4 *__restrict__ copies, uint32_t rows,
+                                                      float4 *__restrict__ grad) {
+    const uint32_t row = blockIdx.x * 8 + threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
+    if (row >= rows) return;
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (uint32_t c = lane; c < kSepCopies; c += kWarp) v = add4(v, copies[(uint64_t)c * rows + row]);
+    v = make_float4(warp_sum(v.x), warp_sum(v.y), warp_sum(v.z), warp_sum(v.w));
+    if (lane == 0 && !is_zero4(v)) red4(reinterpret_cast<float *>(grad + row), v);
+}
+
+// Bytes of the separable gradient's copies behind the other parts of a workspace.
+inline size_t sep_copy_bytes(const qsdvr_render_args *a) {
+    return a->sdf_layers ? (size_t)kSepCopies * (3 * (size_t)a->reso + 1) * sizeof(float4) : 0;
+}
+
 constexpr size_t kCounterBytes = 256;
 static_assert((kLossParts + kWarp) * sizeof(uint32_t) <= kCounterBytes, "counters and partial sums share the area");
 
@@ -1465,6 +1491,7 @@ int launch(const qsdvr_render_args *a, cudaStream_t stream) {
     p.grad_scale = a->grad_scale;
     p.ray_counter = nullptr;
     p.slots = nullptr;
+    p.sep_copies = nullptr;
     p.tlist = a->tlist;
     p.sample_alpha = a->sample_alpha;
     p.sample_capacity = a->sample_capacity;
@@ -1480,7 +1507,13 @@ int launch(const qsdvr_render_args *a, cudaStream_t stream) {
                              (unsigned long long)a->workspace_bytes, kPass == kTrain ? L.train_bytes : L.counter_bytes);
         p.ray_counter = static_cast<uint32_t *>(a->workspace);
         if (kPass == kTrain) p.slots = reinterpret_cast<float *>(static_cast<char *>(a->workspace) + kCounterBytes);
-        const int st = check_cuda(cudaMemsetAsync(p.ray_counter, 0, kPass == kTrain ? kCounterBytes : sizeof(uint32_t), stream), "render: memset");
+        int st = check_cuda(cudaMemsetAsync(p.ray_counter, 0, kPass == kTrain ? kCounterBytes : sizeof(uint32_t), stream),
+                            "render: memset");
+        // (a workspace without room for the copies serves as it did: the REDs go to the caller's table)
+        if (st == QSDVR_OK && kPass != kForward && a->sdf_layers && a->workspace_bytes >= L.train_bytes + sep_copy_bytes(a)) {
+            p.sep_copies = reinterpret_cast<float4 *>(static_cast<char *>(a->workspace) + L.train_bytes);
+            st = check_cuda(cudaMemsetAsync(p.sep_copies, 0, sep_copy_bytes(a), stream), "render: memset");
+        }
         if (st != QSDVR_OK) return st;
         blocks = L.blocks;
     }
@@ -1488,6 +1521,10 @@ int launch(const qsdvr_render_args *a, cudaStream_t stream) {
     qsdvr_render_args variant = *a;
     if (kPass == kForward) variant.merge_scatter = 0;
     dispatch(&variant, launcher);
+    if (p.sep_copies) {
+        const uint32_t rows = 3 * p.R + 1;
+        sep_sum_kernel<<<(rows + 7) / 8, 256, 0, stream>>>(p.sep_copies, rows, p.sep_grad);
+    }
     return check_launch(kPass == kForward ? "qsdvr_render_forward"
                                           : (kPass == kBackward ? "qsdvr_render_backward" : "qsdvr_render_train"));
 }
@@ -1851,7 +1888,7 @@ extern "C" int qsdvr_check_bounds(float *buffer, cudaStream_t stream) {
 extern "C" size_t qsdvr_render_workspace_size(const qsdvr_render_args *args) {
     if (!args) return 0;
     const Layout L = layout_for(args);
-    return L.error == QSDVR_OK ? L.train_bytes : 0;
+    return L.error == QSDVR_OK ? L.train_bytes + sep_copy_bytes(args) : 0;
 }
 
 extern "C" int qsdvr_render_forward(const qsdvr_render_args *args, cudaStream_t stream) {
