@@ -114,19 +114,30 @@ __device__ __forceinline__ float sigmoid(float y) { return 1.0f / (1.0f + __expf
 // (o/8)*SO + (i/8)*128 + (o%8)*16 + (i%8)*2 with SO = kSoW1 (W1) or kSoW2 (W2; its column 64
 // is b2, columns 65..79 zero).  Also the constant features 64..79 (1, 0, ..) of H1 row t, which
 // nothing overwrites.
-__device__ void stage_weights(const __nv_bfloat16 *w, uint8_t *w1s, uint8_t *w2s, uint8_t *hs) {
-    for (int idx = threadIdx.x; idx < 64 * 4; idx += blockDim.x) {  // W1: 64 rows x 4 groups
-        const int o = idx >> 2, g = idx & 3;
-        *reinterpret_cast<uint4 *>(w1s + act_off(o, 8 * g, kSoW1)) =
-            *reinterpret_cast<const uint4 *>(w + o * 32 + 8 * g);
+// All of a thread's loads are issued before its first store: a CTA runs few tiles of a small batch,
+// and eight trips to global memory one after the other were a third of such a launch (the coarse
+// points of 3332 rays 19.8 -> 13.5 us, of 65536 rays 109 -> 101; training on 65536 points 18.4 ->
+// 16.7).
+__device__ __forceinline__ void stage_weights(const __nv_bfloat16 *w, uint8_t *w1s, uint8_t *w2s, uint8_t *hs) {
+    const uint32_t t = threadIdx.x;
+    uint4 r1[2], r2[4];  // W1: 64 rows x 4 groups of 8; W2: 64 rows x 8 groups, and b2 as the ninth
+#pragma unroll
+    for (int k = 0; k < 2; ++k) r1[k] = reinterpret_cast<const uint4 *>(w)[t + kTile * k];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) r2[k] = reinterpret_cast<const uint4 *>(w + kOffW2)[t + kTile * k];
+    const uint32_t b2 = (uint32_t)__bfloat16_as_ushort(w[kOffB2 + (t & 63)]);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const uint32_t i = t + kTile * k;
+        *reinterpret_cast<uint4 *>(w1s + act_off(i >> 2, 8 * (i & 3), kSoW1)) = r1[k];
     }
-    for (int idx = threadIdx.x; idx < 64 * 10; idx += blockDim.x) {  // W2: 64 rows x 10 groups
-        const int o = idx / 10, g = idx % 10;
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (g < 8) v = *reinterpret_cast<const uint4 *>(w + kOffW2 + o * 64 + 8 * g);
-        else if (g == 8) v.x = (uint32_t)__bfloat16_as_ushort(w[kOffB2 + o]);  // (b2[o], 0)
-        *reinterpret_cast<uint4 *>(w2s + act_off(o, 8 * g, kSoW2)) = v;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const uint32_t i = t + kTile * k;
+        *reinterpret_cast<uint4 *>(w2s + act_off(i >> 3, 8 * (i & 7), kSoW2)) = r2[k];
     }
+    // groups 8 (b2[o], 0, ..) by the lower threads and 9 (zeros) by the upper ones
+    *reinterpret_cast<uint4 *>(w2s + act_off(t & 63, t < 64 ? 64 : 72, kSoW2)) = make_uint4(t < 64 ? b2 : 0u, 0, 0, 0);
     const uint32_t one = (uint32_t)__bfloat16_as_ushort(__float2bfloat16(1.0f));
     *reinterpret_cast<uint4 *>(hs + act_off(threadIdx.x, 64, kSpH)) = make_uint4(one, 0, 0, 0);
     *reinterpret_cast<uint4 *>(hs + act_off(threadIdx.x, 72, kSpH)) = make_uint4(0, 0, 0, 0);
@@ -236,7 +247,8 @@ __device__ __forceinline__ void add4_to(float *grad, const float *v, bool vec) {
 // flush, 296 CTAs adding into the same 25 KB.  dw3 is therefore reduced over a warp by exchanging
 // halves (62 shuffles instead of 320) into two registers a lane, added to shared memory once per
 // CTA instead of 64 serial float atomics per warp and tile, and the flush sends 16-byte REDs
-// instead of scalars a row apart: 65536 points 60.5 -> 21 us.
+// instead of scalars a row apart: 65536 points 57.4 -> 18.4 us (16.7 with
+// the weights staged in one round of loads).
 __global__ void __launch_bounds__(128) mlp_train_kernel(const float4 *__restrict__ pts, uint32_t P,
                                                         const __nv_bfloat16 *__restrict__ w, float under_weight,
                                                         float *__restrict__ grad, float *__restrict__ loss_out) {
@@ -443,7 +455,8 @@ __device__ __forceinline__ bool infer_tile_live(const qsdvr_ray_info *__restrict
 // which leaves H1's constant features in place from tile to tile; w3 is read as float4; a tile
 // costs two barriers (a wait that gave up is made block-uniform by the next one, and whether a
 // tile needs the network is read by every thread instead of voted on); and the next tile is
-// encoded while layer 2 runs.  4.2 M points: 108 -> 102.5 us together (the same bits).
+// encoded while layer 2 runs.  4.2 M points: 108 -> 102.5 us together (the same bits; 101 with the
+// weights staged in one round of loads).
 __global__ void __launch_bounds__(128, 6) mlp_infer_kernel(const float4 *__restrict__ pts, uint32_t P,
                                                         const qsdvr_ray_info *__restrict__ rays,
                                                         const float *__restrict__ origin,
@@ -456,16 +469,6 @@ __global__ void __launch_bounds__(128, 6) mlp_infer_kernel(const float4 *__restr
     uint8_t *w2s = w1s + kBytesW1;
     InferSmem &S = *reinterpret_cast<InferSmem *>(w2s + kBytesW2);
     const uint32_t t = threadIdx.x, warp = t >> 5;
-    stage_weights(w, w1s, w2s, buf);
-    if (t < 64) S.w3[t] = bf16f(w, kOffW3 + t);
-    if (t == 0) tc::mbar_init(&S.mbar, 1);
-    if (warp == 0) tc::tmem_alloc(&S.tmem, kInferCols);
-    tc::fence_before_sync();
-    __syncthreads();
-    tc::fence_after_sync();
-    const uint32_t tmem = S.tmem;
-    constexpr uint32_t idesc = tc::idesc_bf16(128, 64, false, false);
-    const float b3 = bf16f(w, kOffB3);
     const uint32_t total = rays ? nrays * 64u : P;
     const uint32_t tiles = (total + kTile - 1) / kTile;
     [[maybe_unused]] const uint64_t extent = rays ? nrays : P;
@@ -492,6 +495,16 @@ __global__ void __launch_bounds__(128, 6) mlp_infer_kernel(const float4 *__restr
     };
     uint32_t phase = 0;
     bool ok = true;  // this thread's waits; made block-uniform at each barrier
+    stage_weights(w, w1s, w2s, buf);
+    if (t < 64) S.w3[t] = bf16f(w, kOffW3 + t);
+    const float b3 = bf16f(w, kOffB3);
+    if (t == 0) tc::mbar_init(&S.mbar, 1);
+    if (warp == 0) tc::tmem_alloc(&S.tmem, kInferCols);
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+    const uint32_t tmem = S.tmem;
+    constexpr uint32_t idesc = tc::idesc_bf16(128, 64, false, false);
     uint32_t tile = next_live(blockIdx.x);
     bool live = false;
     uint32_t x[kF / 2];  // the next tile's features of this thread's point
