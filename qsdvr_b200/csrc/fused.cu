@@ -138,8 +138,8 @@ struct Params {
     float *data_grad;
     float *loss;
     float grad_scale;
-    uint32_t *ray_counter;  // persistent mode: next ray to take (zeroed before the launch), then
-                            // in train mode the warps that are done and the loss's partial sums
+    uint32_t *ray_counter;  // persistent mode: next ray to take, and behind it in train mode the
+                            // loss's partial sums (all zeroed before the launch)
     float *slots;           // persistent train mode: per-warp row stash, kSlotChunks chunks each
     float4 *sep_copies;     // separable gradient: kSepCopies tables that the warps share out, or null
     const float *tlist;     // list sampling: per ray kListT SDF positions (t from origin), or null
@@ -252,6 +252,7 @@ __device__ __forceinline__ void sep_cell(const float4 *sep, uint32_t R, const Ce
 #define QSDVR_SEP_COPIES 64
 #endif
 constexpr uint32_t kSepCopies = QSDVR_SEP_COPIES;
+constexpr uint32_t kSepCopyRays = 4096;  // batches from here on use the copies
 __device__ __forceinline__ void sep_red(float4 *sg, uint32_t R, const CellPoint &c, const float *g) {
     [[maybe_unused]] const uint64_t n = 3ull * R + 1;
     const float4 x = make_float4(g[0], g[3], g[6], 0.0f), y = make_float4(g[1], g[4], g[6], 0.0f),
@@ -945,27 +946,6 @@ __device__ __forceinline__ void backward_chunk(const Params &p, f3 o, f3 d, uint
     __syncwarp();
 }
 
-// The end of a persistent train pass: each warp adds its rays' squared errors (on lane 0) to one
-// of 32 partial sums and the last warp to finish adds those up, so that no sum is a chain of
-// thousands of additions in launch order (one float for all 2368 warps was off by 1e-6; 32 and
-// a tree by 1e-7).  Not inlined: inside the kernel it changed the main loop's register
-// allocation (bf16 degree 3 at 256^3: 2.44 instead of 2.20 ms).
-__device__ __noinline__ void finish_loss(uint32_t *counter, float *loss, float sq, uint32_t warp_id, uint32_t warps) {
-    const int lane = threadIdx.x & 31;
-    float *parts = reinterpret_cast<float *>(counter + kLossParts);
-    uint32_t done = 0;
-    if (lane == 0) {
-        atomicAdd(parts + warp_id % kWarp, sq);
-        asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(done) : "l"(counter + 1) : "memory");
-    }
-    if (__shfl_sync(kFull, done, 0) + 1 == warps) {
-        float v;
-        asm volatile("ld.acquire.gpu.global.f32 %0, [%1];" : "=f"(v) : "l"(parts + lane) : "memory");
-        const float sum = warp_sum(v);
-        if (lane == 0) atomicAdd(loss, sum);
-    }
-}
-
 template <bool kCompat, typename S, int kPass, bool kLogT, int kDeg, int kVar>
 __global__ void __launch_bounds__(kThreads, min_blocks(kPass)) render_kernel(const Params p) {
     constexpr int kRow = Rows<kDeg>::kStride;
@@ -1139,13 +1119,8 @@ __global__ void __launch_bounds__(kThreads, min_blocks(kPass)) render_kernel(con
     }
     if (!persistent) break;
     }  // ray loop
-    if (kPass == kTrain) {
-        if (persistent) {
-            finish_loss(p.ray_counter, p.loss, sq, warp_id, gridDim.x * kWarpsPerBlock);
-        } else if (lane == 0 && sq != 0.0f) {
-            atomicAdd(p.loss, sq);
-        }
-    }
+    if (kPass == kTrain && lane == 0 && sq != 0.0f)
+        atomicAdd(persistent ? reinterpret_cast<float *>(p.ray_counter + kLossParts) + warp_id % kWarp : p.loss, sq);
 }
 
 // ---- TMA brick staging for full frames (forward only, fixed mode, uniform march) --------
@@ -1339,6 +1314,15 @@ __global__ void __launch_bounds__(kBrickThreads) brick_frame_kernel(const __grid
     if (r < p.n) store3(QSDVR_AT(p.color, 3ull * r, 3, 3ull * p.n), acc);
 }
 
+// The loss of a persistent train pass from the 32 partial sums that its warps added to, in a tree,
+// so that no sum is a chain of thousands of additions in launch order (one float for all 2368
+// warps was off by 1e-6, this by 1e-7).  A kernel of its own: 2 us, where the last warp to finish
+// took 6 for it, behind a fence that waited for its gradient REDs.
+__global__ void loss_sum_kernel(const float *__restrict__ parts, float *__restrict__ loss) {
+    const float sum = warp_sum(parts[threadIdx.x]);
+    if (threadIdx.x == 0 && sum != 0.0f) atomicAdd(loss, sum);
+}
+
 // grad[i] += the sum of the copies' entries i, a warp per table row.
 __global__ void __launch_bounds__(256) sep_sum_kernel(const float4 *__restrict__ copies, uint32_t rows,
                                                       float4 *__restrict__ grad) {
@@ -1509,8 +1493,11 @@ int launch(const qsdvr_render_args *a, cudaStream_t stream) {
         if (kPass == kTrain) p.slots = reinterpret_cast<float *>(static_cast<char *>(a->workspace) + kCounterBytes);
         int st = check_cuda(cudaMemsetAsync(p.ray_counter, 0, kPass == kTrain ? kCounterBytes : sizeof(uint32_t), stream),
                             "render: memset");
-        // (a workspace without room for the copies serves as it did: the REDs go to the caller's table)
-        if (st == QSDVR_OK && kPass != kForward && a->sdf_layers && a->workspace_bytes >= L.train_bytes + sep_copy_bytes(a)) {
+        // (a workspace without room for the copies serves as it did: the REDs go to the caller's
+        // table; so they do for short batches, where zeroing and summing the copies costs more than
+        // they save: 2048 rays at 256^3 101 us without and 103 with, 8192 rays 287 and 278)
+        if (st == QSDVR_OK && kPass != kForward && a->sdf_layers && a->ray_count >= kSepCopyRays &&
+            a->workspace_bytes >= L.train_bytes + sep_copy_bytes(a)) {
             p.sep_copies = reinterpret_cast<float4 *>(static_cast<char *>(a->workspace) + L.train_bytes);
             st = check_cuda(cudaMemsetAsync(p.sep_copies, 0, sep_copy_bytes(a), stream), "render: memset");
         }
@@ -1521,6 +1508,8 @@ int launch(const qsdvr_render_args *a, cudaStream_t stream) {
     qsdvr_render_args variant = *a;
     if (kPass == kForward) variant.merge_scatter = 0;
     dispatch(&variant, launcher);
+    if (kPass == kTrain && p.ray_counter)
+        loss_sum_kernel<<<1, kWarp, 0, stream>>>(reinterpret_cast<const float *>(p.ray_counter + kLossParts), p.loss);
     if (p.sep_copies) {
         const uint32_t rows = 3 * p.R + 1;
         sep_sum_kernel<<<(rows + 7) / 8, 256, 0, stream>>>(p.sep_copies, rows, p.sep_grad);

@@ -20,19 +20,19 @@ def test_copies_match_direct(R, passes):
     from qsdvr_b200.camera import Camera
 
     interval, k = 4.0 / 128, 5.0
-    cam = Camera(scenes.look_at((1.8, -3.2, 1.3), 40, 40, 60.0, 2.0, 6.0), interval, R)
-    cam.GenerateRayPoints(torch.ones(1600, dtype=torch.bool))
+    cam = Camera(scenes.look_at((1.8, -3.2, 1.3), 70, 70, 105.0, 2.0, 6.0), interval, R)
+    cam.GenerateRayPoints(torch.ones(4900, dtype=torch.bool))
     g = torch.Generator().manual_seed(R)
     tables = fused.separable_tables(*(1 + 0.05 * torch.randn(R, generator=g).to(DEV) for _ in range(2)),
                                     0.05 * torch.randn(R, generator=g).to(DEV),
                                     torch.tensor([2.0 - 2 * R, 2.0 - 2 * R, R, 0.8 * R * R], device=DEV))
     data = scenes.appearance(R, seed=5).to(DEV)
-    target = torch.rand((1600, 3), generator=g).to(DEV)
+    target = torch.rand((4900, 3), generator=g).to(DEV)
     rays = (cam.rayList, cam.originList, cam.dirList)
-    grad_color = torch.rand((1600, 3), generator=g).to(DEV)
+    grad_color = torch.rand((4900, 3), generator=g).to(DEV)
     outs = []
     for kind in ("copies", "short", "none"):
-        color = torch.zeros((1600, 3), device=DEV)
+        color = torch.zeros((4900, 3), device=DEV)
         tg, dg, loss = torch.zeros_like(tables), torch.zeros_like(data), torch.zeros(1, device=DEV)
         a = fused.make_args(*rays, None, data, R, interval, k, color=color, target=target, grad_color=grad_color,
                             data_grad=dg, loss=loss, grad_scale=0.01, persistent=False, sdf_layers=tables,
