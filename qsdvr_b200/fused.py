@@ -284,26 +284,42 @@ def render_train(target, rays, origin, direction, sdf_grid, data, reso, interval
     return color, loss
 
 
+def gradient_order(rays, origin, direction, interval, data, reso):
+    """``ray_order`` of a batch that is about to be rendered with gradients where that pays, else
+    None.  The order costs about 17 us and shares rows and gradient lines between neighbouring
+    rays in L2, so it pays for grids well above L2 (64 MB: at 64^3 the rows stay in L2 either way)
+    and batches dense enough to have such neighbours.  Forward + backward at 128^3, fp32 degree
+    2: 8192 rays 270 us in batch order, 283 ordered; 16384 rays 461 / 437; 65536 rays 1624 /
+    1277.  At 256^3: 16384 rays 572 / 585, 32768 rays 1062 / 1040, 65536 rays 2051 / 1951."""
+    n = rays.shape[0]
+    if n < 16384 or 2 * n < int(reso) ** 2 or data.numel() * data.element_size() < 64 << 20:
+        return None
+    return ray_order(rays, origin, direction, interval)
+
+
 class FusedRender(autograd.Function):
     """Differentiable fused render.  Forward saves only its inputs; backward recomputes
     each sample's alpha, transmittance and colour (memory O(rays))."""
 
     @staticmethod
     def forward(ctx, sdf_grid, data, rays, origin, direction, reso, interval, k, mode, transmittance):
+        order = None
+        if any(ctx.needs_input_grad[:2]):
+            order = gradient_order(rays, origin, direction, interval, data, reso)
         color = render_forward(rays, origin, direction, sdf_grid.detach(), data.detach(), reso, interval, k, mode,
-                               transmittance)
-        ctx.save_for_backward(sdf_grid, data, rays, origin, direction)
+                               transmittance, order=order)
+        ctx.save_for_backward(sdf_grid, data, rays, origin, direction, order)
         ctx.cfg = (reso, interval, k, mode, transmittance)
         return color
 
     @staticmethod
     def backward(ctx, grad_color):
-        sdf_grid, data, rays, origin, direction = ctx.saved_tensors
+        sdf_grid, data, rays, origin, direction, order = ctx.saved_tensors
         reso, interval, k, mode, transmittance = ctx.cfg
         sg = torch.zeros(sdf_grid.shape, dtype=torch.float32, device=sdf_grid.device)
         dg = torch.zeros(data.shape, dtype=torch.float32, device=data.device)
         render_backward(grad_color, rays, origin, direction, sdf_grid.detach(), data.detach(), reso, interval, k, sg,
-                        dg, mode, transmittance)
+                        dg, mode, transmittance, order=order)
         return sg.to(sdf_grid.dtype), dg.to(data.dtype), None, None, None, None, None, None, None, None
 
 
@@ -402,19 +418,22 @@ class _Bf16Render(autograd.Function):
 
     @staticmethod
     def forward(ctx, sdf_master, data_master, sdf_bf16, data_bf16, rays, origin, direction, model):
-        ctx.save_for_backward(sdf_bf16, data_bf16, rays, origin, direction)
+        order = None
+        if any(ctx.needs_input_grad[:2]):
+            order = gradient_order(rays, origin, direction, model.interval, data_bf16, model.reso)
+        ctx.save_for_backward(sdf_bf16, data_bf16, rays, origin, direction, order)
         ctx.model = model
         return render_forward(rays, origin, direction, sdf_bf16, data_bf16, model.reso, model.interval,
-                              model.logisticCoef, model.mode, model.transmittance)
+                              model.logisticCoef, model.mode, model.transmittance, order=order)
 
     @staticmethod
     def backward(ctx, grad_color):
-        sdf_bf16, data_bf16, rays, origin, direction = ctx.saved_tensors
+        sdf_bf16, data_bf16, rays, origin, direction, order = ctx.saved_tensors
         m = ctx.model
         sg = torch.zeros(sdf_bf16.shape, dtype=torch.float32, device=sdf_bf16.device)
         dg = torch.zeros(data_bf16.shape, dtype=torch.float32, device=data_bf16.device)
         render_backward(grad_color, rays, origin, direction, sdf_bf16, data_bf16, m.reso, m.interval, m.logisticCoef,
-                        sg, dg, m.mode, m.transmittance)
+                        sg, dg, m.mode, m.transmittance, order=order)
         return sg, dg, None, None, None, None, None, None
 
 
@@ -454,20 +473,21 @@ class _SeparableRender(autograd.Function):
     def forward(ctx, x_layer, y_layer, z_layer, offset, data, rays, origin, direction, cfg):
         reso, interval, k, mode, transmittance = cfg
         tables = separable_tables(x_layer.detach(), y_layer.detach(), z_layer.detach(), offset.detach())
+        order = gradient_order(rays, origin, direction, interval, data, reso) if any(ctx.needs_input_grad[:5]) else None
         color = render_forward(rays, origin, direction, None, data.detach(), reso, interval, k, mode, transmittance,
-                               sdf_layers=tables)
-        ctx.save_for_backward(tables, data, rays, origin, direction)
+                               sdf_layers=tables, order=order)
+        ctx.save_for_backward(tables, data, rays, origin, direction, order)
         ctx.cfg = cfg
         return color
 
     @staticmethod
     def backward(ctx, grad_color):
-        tables, data, rays, origin, direction = ctx.saved_tensors
+        tables, data, rays, origin, direction, order = ctx.saved_tensors
         reso, interval, k, mode, transmittance = ctx.cfg
         tg = torch.zeros_like(tables)
         dg = torch.zeros(data.shape, dtype=torch.float32, device=data.device)
         render_backward(grad_color, rays, origin, direction, None, data.detach(), reso, interval, k, tg, dg, mode,
-                        transmittance, sdf_layers=tables)
+                        transmittance, sdf_layers=tables, order=order)
         xg, yg, zg, og = separable_grad(tg)
         return xg, yg, zg, og, dg.to(data.dtype), None, None, None, None
 
@@ -514,7 +534,9 @@ class SeparableRenderGrid(nn.Module):
             self.renderData.grad = torch.zeros_like(self.renderData)
         color, loss = render_train(target, rays, origin, direction, None, self.renderData.detach(), self.reso,
                                    self.interval, self.logisticCoef, tg, self.renderData.grad, self.mode,
-                                   self.transmittance, loss=loss, sdf_layers=tables)
+                                   self.transmittance, loss=loss, sdf_layers=tables,
+                                   order=gradient_order(rays, origin, direction, self.interval, self.renderData,
+                                                        self.reso))
         for p, g in zip((self.xLayer, self.yLayer, self.zLayer, self.offset), separable_grad(tg)):
             p.grad = g if p.grad is None else p.grad.add_(g)
         return color, loss
