@@ -5,8 +5,11 @@ point raises.  There is no CPU or PyTorch fallback.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import os
+
+import torch
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 # QSDVR_B200_LIB selects another build of the library, e.g. DEBUG_LIB_PATH, the bounds-checked
@@ -117,6 +120,21 @@ def call(name: str, *args) -> None:
     status = getattr(lib(), name)(*args)
     if status != OK:
         raise QsdvrError(name, status, lib().qsdvr_last_error().decode(errors="replace"))
+
+
+_NO_GUARD = contextlib.nullcontext()
+
+
+def on_device(dev):
+    """A context with ``dev`` current; nothing to enter when it is already (entering torch's
+    device context costs about 5 us of host time a call)."""
+    return _NO_GUARD if torch.cuda.current_device() == dev.index else torch.cuda.device(dev)
+
+
+def launch(dev, name: str, *args) -> None:
+    """Call an entry point on ``dev`` with torch's current stream there as the last argument."""
+    with on_device(dev):
+        call(name, *args, torch._C._cuda_getCurrentRawStream(dev.index))
 
 
 def size(name: str, *args) -> int:

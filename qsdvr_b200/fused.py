@@ -19,7 +19,7 @@ import torch
 from torch import autograd, nn
 
 from . import _lib
-from ._lib import F32, I32, P, U32, call
+from ._lib import F32, I32, P, U32, launch, on_device
 
 STORAGE = {"f32": 0, "bf16": 1}
 TRANSMITTANCE = {"product": 0, "log": 1}
@@ -150,14 +150,10 @@ def make_args(rays, origin, direction, sdf_grid, data, reso, interval, k, mode="
             raise ValueError(f"order must be a contiguous int32 [N] permutation on {dev}")
         a.order = order.data_ptr()
     if persistent and n:
-        with torch.cuda.device(dev):
+        with on_device(dev):
             ws = workspace(dev, a)
         a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
     return a
-
-
-def _stream(dev):
-    return ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
 
 
 def _check_tlist(tlist, n, dev):
@@ -185,13 +181,12 @@ def ray_order(rays, origin, direction, interval, tlist=None) -> torch.Tensor:
     if ws is None or ws.numel() < need:
         ws = torch.empty(need, dtype=torch.uint8, device=dev)
         _workspaces[key] = ws
-    with torch.cuda.device(dev):
-        if tlist is None:
-            call("qsdvr_ray_order", _ptr(rays), _ptr(origin), _ptr(direction), n, float(interval), _ptr(order),
-                 ws.data_ptr(), ws.numel(), _stream(dev))
-        else:
-            call("qsdvr_ray_order_list", _ptr(rays), _ptr(origin), _ptr(direction), n, _ptr(tlist), _ptr(order),
-                 ws.data_ptr(), ws.numel(), _stream(dev))
+    if tlist is None:
+        launch(dev, "qsdvr_ray_order", _ptr(rays), _ptr(origin), _ptr(direction), n, float(interval), _ptr(order),
+               ws.data_ptr(), ws.numel())
+    else:
+        launch(dev, "qsdvr_ray_order_list", _ptr(rays), _ptr(origin), _ptr(direction), n, _ptr(tlist), _ptr(order),
+               ws.data_ptr(), ws.numel())
     return order
 
 
@@ -199,9 +194,7 @@ def ray_order_keys(rays, origin, direction, interval) -> torch.Tensor:
     """The 30-bit Morton codes of the rays' midpoints (qsdvr_ray_order_keys), int32 [N]."""
     dev, n = _check_batch(rays, origin, direction)
     keys = torch.empty(n, dtype=torch.int32, device=dev)
-    with torch.cuda.device(dev):
-        call("qsdvr_ray_order_keys", _ptr(rays), _ptr(origin), _ptr(direction), n, float(interval), _ptr(keys),
-             _stream(dev))
+    launch(dev, "qsdvr_ray_order_keys", _ptr(rays), _ptr(origin), _ptr(direction), n, float(interval), _ptr(keys))
     return keys
 
 
@@ -218,8 +211,7 @@ def render_forward(rays, origin, direction, sdf_grid, data, reso, interval, k, m
         color = torch.empty((n, 3), dtype=torch.float32, device=dev)
     a = make_args(rays, origin, direction, sdf_grid, data, reso, interval, k, mode, transmittance, color=color,
                   persistent=persistent, tlist=tlist, sample_alpha=sample_alpha, sdf_layers=sdf_layers, order=order)
-    with torch.cuda.device(dev):
-        call("qsdvr_render_forward", ctypes.byref(a), _stream(dev))
+    launch(dev, "qsdvr_render_forward", ctypes.byref(a))
     return color
 
 
@@ -234,8 +226,7 @@ def render_forward_bricks(rays, origin, direction, sdf_grid, data, reso, interva
         color = torch.empty((n, 3), dtype=torch.float32, device=dev)
     a = make_args(rays, origin, direction, sdf_grid, data, reso, interval, k, "fixed", "log", color=color,
                   persistent=False)
-    with torch.cuda.device(dev):
-        call("qsdvr_render_forward_bricks", ctypes.byref(a), _stream(dev))
+    launch(dev, "qsdvr_render_forward_bricks", ctypes.byref(a))
     return color
 
 
@@ -255,8 +246,7 @@ def render_backward(grad_color, rays, origin, direction, sdf_grid, data, reso, i
                   sdf_grad=None if sdf_layers is not None else sdf_grad, data_grad=data_grad,
                   persistent=persistent, tlist=tlist, sdf_layers=sdf_layers,
                   sdf_layers_grad=sdf_grad if sdf_layers is not None else None, order=order, merge=merge)
-    with torch.cuda.device(dev):
-        call("qsdvr_render_backward", ctypes.byref(a), _stream(dev))
+    launch(dev, "qsdvr_render_backward", ctypes.byref(a))
 
 
 def render_train(target, rays, origin, direction, sdf_grid, data, reso, interval, k, sdf_grad, data_grad,
@@ -279,8 +269,7 @@ def render_train(target, rays, origin, direction, sdf_grid, data, reso, interval
                   grad_scale=2.0 / (3.0 * max(n, 1)), persistent=persistent, tlist=tlist,
                   sample_alpha=sample_alpha, sdf_layers=sdf_layers, sdf_layers_grad=sdf_grad if sep else None,
                   order=order, merge=merge)
-    with torch.cuda.device(dev):
-        call("qsdvr_render_train", ctypes.byref(a), _stream(dev))
+    launch(dev, "qsdvr_render_train", ctypes.byref(a))
     return color, loss
 
 
@@ -335,8 +324,7 @@ def sdf_cells_bf16(grid8: torch.Tensor, out: torch.Tensor | None = None) -> torc
     elif out.dtype != torch.bfloat16 or out.shape != grid8.shape or out.device != grid8.device \
             or not out.is_contiguous():
         raise ValueError("out must be a contiguous bfloat16 tensor shaped like grid8")
-    with torch.cuda.device(grid8.device):
-        call("qsdvr_sdf_cells_bf16", _ptr(grid8), _ptr(out), grid8.shape[0], _stream(grid8.device))
+    launch(grid8.device, "qsdvr_sdf_cells_bf16", _ptr(grid8), _ptr(out), grid8.shape[0])
     return out
 
 
@@ -448,9 +436,7 @@ def separable_tables(x_layer, y_layer, z_layer, offset) -> torch.Tensor:
         if not t.is_cuda or t.device != dev or t.dtype != torch.float32 or t.numel() != nn_ or not t.is_contiguous():
             raise ValueError(f"{nm} must be a contiguous float32 CUDA tensor of {nn_} values on {dev}")
     out = torch.empty((3 * R + 1, 4), dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
-        call("qsdvr_separable_sdf_tables", _ptr(x_layer), _ptr(y_layer), _ptr(z_layer), _ptr(offset), R, _ptr(out),
-             _stream(dev))
+    launch(dev, "qsdvr_separable_sdf_tables", _ptr(x_layer), _ptr(y_layer), _ptr(z_layer), _ptr(offset), R, _ptr(out))
     return out
 
 
@@ -463,8 +449,7 @@ def separable_grad(table_grad: torch.Tensor):
         raise ValueError("table_grad must be a contiguous float32 [3R+1,4] tensor")
     xg, yg, zg = (torch.empty(R, dtype=torch.float32, device=dev) for _ in range(3))
     og = torch.empty(4, dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
-        call("qsdvr_separable_sdf_grad", _ptr(table_grad), R, _ptr(xg), _ptr(yg), _ptr(zg), _ptr(og), _stream(dev))
+    launch(dev, "qsdvr_separable_sdf_grad", _ptr(table_grad), R, _ptr(xg), _ptr(yg), _ptr(zg), _ptr(og))
     return xg, yg, zg, og
 
 

@@ -20,7 +20,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from ._lib import call
+from ._lib import launch, on_device
 
 __all__ = ["CameraArgs", "GridInterpolationForward", "GridInterpolationBackward", "LayerToGridForward",
            "LayerToGridBackward", "SampleSDFForward", "SampleSDFBackward", "SampleNormalForward",
@@ -101,10 +101,6 @@ def _p(t) -> ctypes.c_void_p:
     return ctypes.c_void_p(t.data_ptr() if t is not None and t.numel() else 0)
 
 
-def _stream(device) -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
-
-
 def _rows(t, name, width, device, dtype=torch.float32):
     _check(t, name, dtype, device)
     if t.numel() % width:
@@ -122,9 +118,8 @@ def GridInterpolationForward(dataGrid, pointList, indexList, out, reso):
     _check(out, "out", torch.float32, dev)
     if dataGrid.shape[-1] != 32 or out.numel() != 32 * n:
         raise ValueError("GridInterpolationForward: 32 channels per vertex and out of [N,32] expected")
-    with torch.cuda.device(dev):
-        call("qsdvr_grid_interpolation_forward", _p(dataGrid), _p(pointList), _p(indexList), _p(out), n, int(reso),
-             dataGrid.numel() // 32, _stream(dev))
+    launch(dev, "qsdvr_grid_interpolation_forward", _p(dataGrid), _p(pointList), _p(indexList), _p(out), n, int(reso),
+           dataGrid.numel() // 32)
 
 
 def GridInterpolationBackward(dataGrid, pointList, indexList, out, reso):
@@ -135,9 +130,8 @@ def GridInterpolationBackward(dataGrid, pointList, indexList, out, reso):
     _check(out, "out", torch.float32, dev)
     if dataGrid.shape[-1] != 32 or out.numel() != 32 * n:
         raise ValueError("GridInterpolationBackward: 32 channels per vertex and gradient of [N,32] expected")
-    with torch.cuda.device(dev):
-        call("qsdvr_grid_interpolation_backward", _p(dataGrid), _p(pointList), _p(indexList), _p(out), n, int(reso),
-             dataGrid.numel() // 32, _stream(dev))
+    launch(dev, "qsdvr_grid_interpolation_backward", _p(dataGrid), _p(pointList), _p(indexList), _p(out), n, int(reso),
+           dataGrid.numel() // 32)
 
 
 def ShaderForward(out, normalList, viewDirList, dataList, specularList, *, mode="compat"):
@@ -149,9 +143,8 @@ def ShaderForward(out, normalList, viewDirList, dataList, specularList, *, mode=
             raise ValueError(f"ShaderForward: {nm} has {t.numel() // 3} rows, expected {n}")
     if _rows(dataList, "dataList", 32, dev) != n:
         raise ValueError("ShaderForward: dataList must be [N,32]")
-    with torch.cuda.device(dev):
-        call("qsdvr_shader_forward", _p(out), _p(normalList), _p(viewDirList), _p(dataList), _p(specularList), n,
-             _MODES[mode], _stream(dev))
+    launch(dev, "qsdvr_shader_forward", _p(out), _p(normalList), _p(viewDirList), _p(dataList), _p(specularList), n,
+           _MODES[mode])
 
 
 def ShaderBackward(out, normalList, viewDirList, dataList, specularList, normalGradList, dataGradList, *,
@@ -165,9 +158,8 @@ def ShaderBackward(out, normalList, viewDirList, dataList, specularList, normalG
             raise ValueError(f"ShaderBackward: {nm} has {t.numel() // 3} rows, expected {n}")
     if _rows(dataList, "dataList", 32, dev) != n or _rows(dataGradList, "dataGradList", 32, dev) != n:
         raise ValueError("ShaderBackward: dataList/dataGradList must be [N,32]")
-    with torch.cuda.device(dev):
-        call("qsdvr_shader_backward", _p(out), _p(normalList), _p(viewDirList), _p(dataList), _p(specularList),
-             _p(normalGradList), _p(dataGradList), n, _MODES[mode], _stream(dev))
+    launch(dev, "qsdvr_shader_backward", _p(out), _p(normalList), _p(viewDirList), _p(dataList), _p(specularList),
+           _p(normalGradList), _p(dataGradList), n, _MODES[mode])
 
 
 def _rays(rayList, dev):
@@ -185,9 +177,8 @@ def RayAggregateForward(out, rgbList, sdfList, rayList, alphaList, TList, logist
     s = _rows(sdfList, "sdfList", 1, dev)
     if _rows(out, "out", 3, dev) != nr or _rows(alphaList, "alphaList", 1, dev) < m or _rows(TList, "TList", 1, dev) < m:
         raise ValueError("RayAggregateForward: out must be [N,3], alphaList/TList as long as rgbList")
-    with torch.cuda.device(dev):
-        call("qsdvr_ray_aggregate_forward", _p(out), _p(rgbList), _p(sdfList), _p(rayList), _p(alphaList), _p(TList),
-             nr, float(logisticCoef), s, m, _stream(dev))
+    launch(dev, "qsdvr_ray_aggregate_forward", _p(out), _p(rgbList), _p(sdfList), _p(rayList), _p(alphaList), _p(TList),
+           nr, float(logisticCoef), s, m)
 
 
 def RayAggregateBackward(outgrad, rgbList, sdfList, rayList, alphaList, TList, rgbGradList, sdfGradList,
@@ -201,9 +192,8 @@ def RayAggregateBackward(outgrad, rgbList, sdfList, rayList, alphaList, TList, r
             or _rows(sdfGradList, "sdfGradList", 1, dev) != s or _rows(alphaList, "alphaList", 1, dev) < m
             or _rows(TList, "TList", 1, dev) < m):
         raise ValueError("RayAggregateBackward: inconsistent shapes")
-    with torch.cuda.device(dev):
-        call("qsdvr_ray_aggregate_backward", _p(outgrad), _p(rgbList), _p(sdfList), _p(rayList), _p(alphaList),
-             _p(TList), _p(rgbGradList), _p(sdfGradList), nr, float(logisticCoef), s, m, _stream(dev))
+    launch(dev, "qsdvr_ray_aggregate_backward", _p(outgrad), _p(rgbList), _p(sdfList), _p(rayList), _p(alphaList),
+           _p(TList), _p(rgbGradList), _p(sdfGradList), nr, float(logisticCoef), s, m)
 
 
 # ----------------------------------------------------------------------------- surface.cu
@@ -223,9 +213,7 @@ def SampleSDFForward(out, sdfGrid, pointList, indexList, reso):
     _check(indexList, "indexList", torch.int32, dev, (n,))
     if _rows(out, "out", 1, dev) != n:
         raise ValueError("SampleSDFForward: out must have one value per point")
-    with torch.cuda.device(dev):
-        call("qsdvr_sample_sdf_forward", _p(out), _p(sdfGrid), _p(pointList), _p(indexList), n, float(reso), cells,
-             _stream(dev))
+    launch(dev, "qsdvr_sample_sdf_forward", _p(out), _p(sdfGrid), _p(pointList), _p(indexList), n, float(reso), cells)
 
 
 def SampleSDFBackward(out, sdfGrid, pointList, indexList, sdfGradGrid, reso):
@@ -238,9 +226,8 @@ def SampleSDFBackward(out, sdfGrid, pointList, indexList, sdfGradGrid, reso):
     _check(indexList, "indexList", torch.int32, dev, (n,))
     if _rows(out, "out", 1, dev) != n:
         raise ValueError("SampleSDFBackward: gradient must have one value per point")
-    with torch.cuda.device(dev):
-        call("qsdvr_sample_sdf_backward", _p(out), _p(sdfGrid), _p(pointList), _p(indexList), _p(sdfGradGrid), n,
-             float(reso), cells, _stream(dev))
+    launch(dev, "qsdvr_sample_sdf_backward", _p(out), _p(sdfGrid), _p(pointList), _p(indexList), _p(sdfGradGrid), n,
+           float(reso), cells)
 
 
 def SampleNormalForward(out, sdfGrid, pointList, indexList):
@@ -251,9 +238,7 @@ def SampleNormalForward(out, sdfGrid, pointList, indexList):
     _check(indexList, "indexList", torch.int32, dev, (n,))
     if _rows(out, "out", 3, dev) != n:
         raise ValueError("SampleNormalForward: out must be [N,3]")
-    with torch.cuda.device(dev):
-        call("qsdvr_sample_normal_forward", _p(out), _p(sdfGrid), _p(pointList), _p(indexList), n, cells,
-             _stream(dev))
+    launch(dev, "qsdvr_sample_normal_forward", _p(out), _p(sdfGrid), _p(pointList), _p(indexList), n, cells)
 
 
 def SampleNormalBackward(out, sdfGrid, pointList, indexList, sdfGradGrid):
@@ -266,9 +251,8 @@ def SampleNormalBackward(out, sdfGrid, pointList, indexList, sdfGradGrid):
     _check(indexList, "indexList", torch.int32, dev, (n,))
     if _rows(out, "out", 3, dev) != n:
         raise ValueError("SampleNormalBackward: gradient must be [N,3]")
-    with torch.cuda.device(dev):
-        call("qsdvr_sample_normal_backward", _p(out), _p(sdfGrid), _p(pointList), _p(indexList), _p(sdfGradGrid), n,
-             cells, _stream(dev))
+    launch(dev, "qsdvr_sample_normal_backward", _p(out), _p(sdfGrid), _p(pointList), _p(indexList), _p(sdfGradGrid), n,
+           cells)
 
 
 def LayerToGridForward(out, xLayer, yLayer, zLayer, offset):
@@ -279,12 +263,16 @@ def LayerToGridForward(out, xLayer, yLayer, zLayer, offset):
         raise ValueError("LayerToGridForward: out [R,R,R,7], three layers [R] and offset [4] expected")
     for t, nm in ((xLayer, "xLayer"), (yLayer, "yLayer"), (zLayer, "zLayer"), (offset, "offset")):
         _check(t, nm, torch.float32, cuda=False)
-    with torch.cuda.device(dev):
-        x, y, z = (t.to(dev, non_blocking=True) for t in (xLayer, yLayer, zLayer))
-        off = offset.reshape(-1)[:4].to(dev, non_blocking=True).contiguous()
+    with on_device(dev):
+        if not any(t.is_cuda or t.is_pinned() for t in (xLayer, yLayer, zLayer, offset)):
+            # pageable host layers (the reference's) cross in one copy instead of four
+            x, y, z, off = torch.cat([xLayer.reshape(-1), yLayer.reshape(-1), zLayer.reshape(-1),
+                                      offset.reshape(-1)[:4]]).to(dev).split((R, R, R, 4))
+        else:
+            x, y, z = (t.to(dev, non_blocking=True) for t in (xLayer, yLayer, zLayer))
+            off = offset.reshape(-1)[:4].to(dev, non_blocking=True).contiguous()
         ws = torch.empty(_lib.size("qsdvr_layer_to_grid_workspace_size", R), dtype=torch.uint8, device=dev)
-        call("qsdvr_layer_to_grid_forward", _p(out), _p(x), _p(y), _p(z), _p(off), R, _p(ws), ws.numel(),
-             _stream(dev))
+        launch(dev, "qsdvr_layer_to_grid_forward", _p(out), _p(x), _p(y), _p(z), _p(off), R, _p(ws), ws.numel())
 
 
 def LayerToGridBackward(out, xLayer, yLayer, zLayer, offset):
@@ -294,11 +282,13 @@ def LayerToGridBackward(out, xLayer, yLayer, zLayer, offset):
     R = xLayer.numel()
     if out.numel() != R ** 3 * 7 or yLayer.numel() != R or zLayer.numel() != R or offset.numel() < 4:
         raise ValueError("LayerToGridBackward: gradient [R,R,R,7], three layers [R] and offset [4] expected")
-    with torch.cuda.device(dev):
+    with on_device(dev):
         g = torch.empty(3 * R + 4, dtype=torch.float32, device=dev)
         ws = torch.empty(_lib.size("qsdvr_layer_to_grid_workspace_size", R), dtype=torch.uint8, device=dev)
-        call("qsdvr_layer_to_grid_backward", _p(out), R, _p(g[:R]), _p(g[R:2 * R]), _p(g[2 * R:3 * R]),
-             _p(g[3 * R:]), _p(ws), ws.numel(), _stream(dev))
+        launch(dev, "qsdvr_layer_to_grid_backward", _p(out), R, _p(g[:R]), _p(g[R:2 * R]), _p(g[2 * R:3 * R]),
+               _p(g[3 * R:]), _p(ws), ws.numel())
+        if all(not t.is_cuda for t in (xLayer, yLayer, zLayer, offset)):
+            g = g.cpu()  # host layers: one copy and one wait
         xLayer.copy_(g[:R].view_as(xLayer))
         yLayer.copy_(g[R:2 * R].view_as(yLayer))
         zLayer.copy_(g[2 * R:3 * R].view_as(zLayer))
@@ -318,12 +308,12 @@ def RayCut(args: CameraArgs, mask, rayList, originList, dirList, interval):
     if originList.numel() < 3 * P or dirList.numel() < 3 * P or mask.numel() < P:
         raise ValueError("RayCut: originList/dirList need [pixelCount,3], mask [pixelCount]")
     cam = args.to_c()
-    with torch.cuda.device(dev):
+    with on_device(dev):
         m = mask.reshape(-1)[:P].to(dev, torch.uint8, non_blocking=True).contiguous()
         ws = torch.empty(_lib.size("qsdvr_ray_cut_workspace_size", P), dtype=torch.uint8, device=dev)
         totals = torch.empty(2, dtype=torch.int32, device=dev)
-        call("qsdvr_ray_cut", ctypes.byref(cam), _p(m), _p(rayList), _p(originList), _p(dirList), float(interval), P,
-             _p(totals), _p(ws), ws.numel(), _stream(dev))
+        launch(dev, "qsdvr_ray_cut", ctypes.byref(cam), _p(m), _p(rayList), _p(originList), _p(dirList),
+               float(interval), P, _p(totals), _p(ws), ws.numel())
         t = totals.cpu()
     args.sdfCount = int(t[0])
     args.renderCount = int(t[1])
@@ -342,7 +332,6 @@ def GenerateRayPoints(args, sdfPointList, sdfIndexList, renderPointList, renderI
     _check(renderIndexList, "renderIndexList", torch.int32, dev, (m,))
     if _rows(viewDirList, "viewDirList", 3, dev) != m:
         raise ValueError("GenerateRayPoints: viewDirList must match renderPointList")
-    with torch.cuda.device(dev):
-        call("qsdvr_generate_ray_points", _p(rayList), _p(originList), _p(dirList), n, float(interval),
-             int(baseVolumeReso), _p(sdfPointList), _p(sdfIndexList), _p(renderPointList), _p(renderIndexList),
-             _p(viewDirList), s, m, _stream(dev))
+    launch(dev, "qsdvr_generate_ray_points", _p(rayList), _p(originList), _p(dirList), n, float(interval),
+           int(baseVolumeReso), _p(sdfPointList), _p(sdfIndexList), _p(renderPointList), _p(renderIndexList),
+           _p(viewDirList), s, m)
