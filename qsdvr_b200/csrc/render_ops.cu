@@ -90,14 +90,53 @@ __global__ void __launch_bounds__(256) interp_backward_kernel(float *__restrict_
 
 // ---- shader (kernel/render.cu:154-221) -------------------------------------------------------
 
+// A thread reads, and in the backward writes, a whole row.  There 32-byte accesses, where the
+// buffers are aligned for them (kWide), move each sector in one piece: 1.3 M samples 84 -> 66 us.
+// (The forward, which only reads, and the interpolation stayed at 40 us and went from 104 to 116
+// with them: they keep the 16-byte ones.)
+struct Chunk8 {
+    float4 lo, hi;
+};
+template <bool kWide>
+__device__ __forceinline__ Chunk8 ld_chunk(const float *p) {
+    Chunk8 r;
+    if (kWide) {
+        asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=f"(r.lo.x), "=f"(r.lo.y), "=f"(r.lo.z), "=f"(r.lo.w), "=f"(r.hi.x), "=f"(r.hi.y), "=f"(r.hi.z),
+                       "=f"(r.hi.w)
+                     : "l"(p));
+    } else {
+        r.lo = ld4(p);
+        r.hi = ld4(p + 4);
+    }
+    return r;
+}
+template <bool kWide>
+__device__ __forceinline__ void st_chunk(float *p, float4 lo, float4 hi) {
+    if (kWide) {
+        asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(lo.x), "f"(lo.y), "f"(lo.z),
+                     "f"(lo.w), "f"(hi.x), "f"(hi.y), "f"(hi.z), "f"(hi.w)
+                     : "memory");
+    } else {
+        st4(p, lo);
+        st4(p + 4, hi);
+    }
+}
+
+
+template <bool kWide>
 __device__ __forceinline__ void load_row(const float *p, float *d) {
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        const float4 v = ld4(p + 4 * k);
-        d[4 * k] = v.x;
-        d[4 * k + 1] = v.y;
-        d[4 * k + 2] = v.z;
-        d[4 * k + 3] = v.w;
+    for (int k = 0; k < kC; k += 8) {
+        const Chunk8 v = ld_chunk<kWide>(p + k);
+        d[k] = v.lo.x;
+        d[k + 1] = v.lo.y;
+        d[k + 2] = v.lo.z;
+        d[k + 3] = v.lo.w;
+        d[k + 4] = v.hi.x;
+        d[k + 5] = v.hi.y;
+        d[k + 6] = v.hi.z;
+        d[k + 7] = v.hi.w;
     }
 }
 
@@ -109,14 +148,14 @@ __global__ void __launch_bounds__(128) shader_forward_kernel(float *__restrict__
     const uint64_t id = blockIdx.x * 128ull + threadIdx.x;
     if (id >= n) return;
     float d[kC];
-    load_row(data + id * kC, d);
+    load_row<false>(data + id * kC, d);
     f3 spec;
     const f3 rgb = shade<kCompat>(load3(nrm + 3 * id), load3(view + 3 * id), d, &spec);
     store3(out + 3 * id, rgb);
     store3(spec_out + 3 * id, spec);
 }
 
-template <bool kCompat>
+template <bool kCompat, bool kWide>
 __global__ void __launch_bounds__(128) shader_backward_kernel(const float *__restrict__ gout,
                                                               const float *__restrict__ nrm,
                                                               const float *__restrict__ view,
@@ -127,12 +166,14 @@ __global__ void __launch_bounds__(128) shader_backward_kernel(const float *__res
     const uint64_t id = blockIdx.x * 128ull + threadIdx.x;
     if (id >= n) return;
     float d[kC], g[kC];
-    load_row(data + id * kC, d);
+    load_row<kWide>(data + id * kC, d);
     const f3 ng = shade_backward<kCompat>(load3(gout + 3 * id), load3(nrm + 3 * id), load3(view + 3 * id), d,
                                           load3(spec + 3 * id), g);
     store3(ngrad + 3 * id, ng);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) st4(dgrad + id * kC + 4 * k, make_float4(g[4 * k], g[4 * k + 1], g[4 * k + 2], g[4 * k + 3]));
+    for (int k = 0; k < kC; k += 8)
+        st_chunk<kWide>(dgrad + id * kC + k, make_float4(g[k], g[k + 1], g[k + 2], g[k + 3]),
+                        make_float4(g[k + 4], g[k + 5], g[k + 6], g[k + 7]));
 }
 
 // ---- compositing (kernel/render.cu:223-315) ----------------------------------------------
@@ -341,12 +382,13 @@ extern "C" int qsdvr_shader_backward(const float *grad_out, const float *normal,
         return set_error(QSDVR_ERR_INVALID_ARGUMENT, "qsdvr_shader_backward: bad mode %d", mode);
     if (!aligned(data, 16) || !aligned(data_grad, 16))
         return set_error(QSDVR_ERR_ALIGNMENT, "qsdvr_shader_backward: data buffers need 16-byte alignment");
-    if (mode == QSDVR_MODE_COMPAT)
-        shader_backward_kernel<true><<<grid_for(count, 128), 128, 0, stream>>>(grad_out, normal, view, data, specular,
-                                                                              normal_grad, data_grad, count);
-    else
-        shader_backward_kernel<false><<<grid_for(count, 128), 128, 0, stream>>>(grad_out, normal, view, data, specular,
-                                                                               normal_grad, data_grad, count);
+    const bool wide = aligned(data, 32) && aligned(data_grad, 32);
+    auto run = [&](auto kernel) {
+        kernel<<<grid_for(count, 128), 128, 0, stream>>>(grad_out, normal, view, data, specular, normal_grad, data_grad,
+                                                         count);
+    };
+    if (mode == QSDVR_MODE_COMPAT) wide ? run(shader_backward_kernel<true, true>) : run(shader_backward_kernel<true, false>);
+    else wide ? run(shader_backward_kernel<false, true>) : run(shader_backward_kernel<false, false>);
     return check_launch("qsdvr_shader_backward");
 }
 
