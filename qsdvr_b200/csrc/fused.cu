@@ -1606,17 +1606,19 @@ constexpr uint32_t kOrderBuckets = (1u << 15) + 1;
 // With a sample list (list mode) the key point is each ray's median SDF position instead: the
 // fine samples gather where the compositing weights are, so rays keyed there run beside the
 // rays that hit the same patch of the surface and share its vertex rows and gradient lines.
+// Two kernels compute it and have to agree, so every operation is rounded explicitly.
 __device__ __forceinline__ uint32_t ray_bucket(const qsdvr_ray_info *rays, const float *origin, const float *dir,
                                                uint32_t r, uint32_t n, float interval, const float *tlist) {
     const uint32_t ns = rays[r].sdf_count;
     if (ns < 2) return kOrderBuckets - 1;
     const float t = tlist ? *QSDVR_AT(tlist, (uint64_t)kListT * r + kListT / 2, 1, (uint64_t)kListT * n)
-                          : 0.5f * (float)(ns - 1) * interval;
+                          : __fmul_rn(__fmul_rn(0.5f, (float)(ns - 1)), interval);
     const f3 o = load3(origin + 3ull * r), d = load3(dir + 3ull * r);
-    const float c[3] = {fmaf(d.x, t, o.x), fmaf(d.y, t, o.y), fmaf(d.z, t, o.z)};
+    const float c[3] = {__fmaf_rn(d.x, t, o.x), __fmaf_rn(d.y, t, o.y), __fmaf_rn(d.z, t, o.z)};
     uint32_t q[3];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) q[a] = (uint32_t)fminf(fmaxf((c[a] + 1.0f) * 16.0f, 0.0f), 31.0f);
+    for (int a = 0; a < 3; ++a)
+        q[a] = (uint32_t)fminf(fmaxf(__fmul_rn(__fadd_rn(c[a], 1.0f), 16.0f), 0.0f), 31.0f);
     return spread3(q[0]) | (spread3(q[1]) << 1) | (spread3(q[2]) << 2);
 }
 

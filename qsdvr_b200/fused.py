@@ -286,15 +286,20 @@ def gradient_order(rays, origin, direction, interval, data, reso):
     return ray_order(rays, origin, direction, interval)
 
 
+def _module_order(params, rays, origin, direction, interval, data, reso):
+    """``gradient_order`` for a module's render, where gradients will be taken (an autograd function's
+    own forward cannot see torch.no_grad, and a frame rendered without gradients needs no order)."""
+    if not (torch.is_grad_enabled() and any(p.requires_grad for p in params)):
+        return None
+    return gradient_order(rays, origin, direction, interval, data, reso)
+
+
 class FusedRender(autograd.Function):
     """Differentiable fused render.  Forward saves only its inputs; backward recomputes
     each sample's alpha, transmittance and colour (memory O(rays))."""
 
     @staticmethod
-    def forward(ctx, sdf_grid, data, rays, origin, direction, reso, interval, k, mode, transmittance):
-        order = None
-        if any(ctx.needs_input_grad[:2]):
-            order = gradient_order(rays, origin, direction, interval, data, reso)
+    def forward(ctx, sdf_grid, data, rays, origin, direction, reso, interval, k, mode, transmittance, order=None):
         color = render_forward(rays, origin, direction, sdf_grid.detach(), data.detach(), reso, interval, k, mode,
                                transmittance, order=order)
         ctx.save_for_backward(sdf_grid, data, rays, origin, direction, order)
@@ -309,7 +314,7 @@ class FusedRender(autograd.Function):
         dg = torch.zeros(data.shape, dtype=torch.float32, device=data.device)
         render_backward(grad_color, rays, origin, direction, sdf_grid.detach(), data.detach(), reso, interval, k, sg,
                         dg, mode, transmittance, order=order)
-        return sg.to(sdf_grid.dtype), dg.to(data.dtype), None, None, None, None, None, None, None, None
+        return sg.to(sdf_grid.dtype), dg.to(data.dtype), None, None, None, None, None, None, None, None, None
 
 
 def sdf_cells_bf16(grid8: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
@@ -391,11 +396,13 @@ class DenseRenderGrid(nn.Module):
         return self.sdfGrid, self.renderData
 
     def forward(self, rays, origin, direction):
+        order = _module_order((self.sdfGrid, self.renderData), rays, origin, direction, self.interval, self.grids()[1],
+                              self.reso)
         if self.storage == "bf16":
             return _Bf16Render.apply(self.sdfGrid, self.renderData, self._copies[0], self._copies[1], rays, origin,
-                                     direction, self)
+                                     direction, self, order)
         return FusedRender.apply(self.sdfGrid, self.renderData, rays, origin, direction, self.reso, self.interval,
-                                 self.logisticCoef, self.mode, self.transmittance)
+                                 self.logisticCoef, self.mode, self.transmittance, order)
 
     def set_logisticCoef(self, logisticCoef):
         self.logisticCoef = logisticCoef
@@ -405,10 +412,7 @@ class _Bf16Render(autograd.Function):
     """Forward/backward on the bf16 copies; gradients (fp32) flow to the fp32 masters."""
 
     @staticmethod
-    def forward(ctx, sdf_master, data_master, sdf_bf16, data_bf16, rays, origin, direction, model):
-        order = None
-        if any(ctx.needs_input_grad[:2]):
-            order = gradient_order(rays, origin, direction, model.interval, data_bf16, model.reso)
+    def forward(ctx, sdf_master, data_master, sdf_bf16, data_bf16, rays, origin, direction, model, order):
         ctx.save_for_backward(sdf_bf16, data_bf16, rays, origin, direction, order)
         ctx.model = model
         return render_forward(rays, origin, direction, sdf_bf16, data_bf16, model.reso, model.interval,
@@ -422,7 +426,7 @@ class _Bf16Render(autograd.Function):
         dg = torch.zeros(data_bf16.shape, dtype=torch.float32, device=data_bf16.device)
         render_backward(grad_color, rays, origin, direction, sdf_bf16, data_bf16, m.reso, m.interval, m.logisticCoef,
                         sg, dg, m.mode, m.transmittance, order=order)
-        return sg, dg, None, None, None, None, None, None
+        return sg, dg, None, None, None, None, None, None, None
 
 
 # ----------------------------------------------------------------------------- separable SDF
@@ -455,10 +459,9 @@ def separable_grad(table_grad: torch.Tensor):
 
 class _SeparableRender(autograd.Function):
     @staticmethod
-    def forward(ctx, x_layer, y_layer, z_layer, offset, data, rays, origin, direction, cfg):
+    def forward(ctx, x_layer, y_layer, z_layer, offset, data, rays, origin, direction, cfg, order):
         reso, interval, k, mode, transmittance = cfg
         tables = separable_tables(x_layer.detach(), y_layer.detach(), z_layer.detach(), offset.detach())
-        order = gradient_order(rays, origin, direction, interval, data, reso) if any(ctx.needs_input_grad[:5]) else None
         color = render_forward(rays, origin, direction, None, data.detach(), reso, interval, k, mode, transmittance,
                                sdf_layers=tables, order=order)
         ctx.save_for_backward(tables, data, rays, origin, direction, order)
@@ -474,7 +477,7 @@ class _SeparableRender(autograd.Function):
         render_backward(grad_color, rays, origin, direction, None, data.detach(), reso, interval, k, tg, dg, mode,
                         transmittance, sdf_layers=tables, order=order)
         xg, yg, zg, og = separable_grad(tg)
-        return xg, yg, zg, og, dg.to(data.dtype), None, None, None, None
+        return xg, yg, zg, og, dg.to(data.dtype), None, None, None, None, None
 
 
 class SeparableRenderGrid(nn.Module):
@@ -506,8 +509,9 @@ class SeparableRenderGrid(nn.Module):
         return (self.reso, self.interval, self.logisticCoef, self.mode, self.transmittance)
 
     def forward(self, rays, origin, direction):
+        order = _module_order(self.parameters(), rays, origin, direction, self.interval, self.renderData, self.reso)
         return _SeparableRender.apply(self.xLayer, self.yLayer, self.zLayer, self.offset, self.renderData, rays, origin,
-                                      direction, self.cfg())
+                                      direction, self.cfg(), order)
 
     def train_step(self, target, rays, origin, direction, loss=None):
         """Forward + MSE + backward in one fused launch; accumulates into the parameters' .grad.

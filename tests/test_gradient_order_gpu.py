@@ -59,6 +59,7 @@ def test_ordered_gradients_match_batch_order(model, monkeypatch):
     assert torch.equal(outs[0][0], outs[1][0])
     for a, b in zip(outs[0][1:], outs[1][1:]):
         assert a.abs().max() > 0 and rel_err(a.cpu(), b.cpu()) < 1e-5
+    monkeypatch.setattr(fused, "gradient_order", noting)
     with torch.no_grad():  # no gradients, no order
-        m(*rays)
+        assert torch.equal(m(*rays), outs[0][0])
     assert seen == [True]
