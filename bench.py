@@ -462,7 +462,7 @@ def run_ours(args, cfg, device, ws, rank):
                    "l2": "inputs larger than L2 (grids 2.7 GB), no flush", "parallelism": f"replicas x{ws}"},
         "e2e": {"value": round(e2e_value, 1), "unit": "rays/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": 4,
                 "wall_s": round(wall_e2e, 3)},
-        "gpu_launches": 4 * args.steps,  # qsdvr_ray_order's 3 kernels + the train kernel per step
+        "gpu_launches": 5 * args.steps,  # qsdvr_ray_order's 3 kernels, the train kernel and its loss sum per step
         "step_parts": step_parts,
         "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                      "frac": round(achieved / peak, 4), "traffic": None if traffic is None else round(traffic),
