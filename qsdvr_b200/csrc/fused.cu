@@ -85,14 +85,6 @@ constexpr uint32_t kSlotChunks = QSDVR_SLOT_CHUNKS;
 #ifndef QSDVR_STASH_DISCARD
 #define QSDVR_STASH_DISCARD 1
 #endif
-// Latency: the gather walks a chunk's samples a few at a time, and each round of its loads
-// waited for DRAM.  With QSDVR_GATHER_PREFETCH every shaded sample beyond the first round
-// requests its 8 corner rows into L2 (four bulk prefetches of two adjacent rows) as soon as
-// the chunk's alpha is known, so the later rounds find them there: SH degree 2 only (1, the
-// default: with 64-channel rows the prefetches measured slower), every degree (2), none (0).
-#ifndef QSDVR_GATHER_PREFETCH
-#define QSDVR_GATHER_PREFETCH 1
-#endif
 template <int kDeg>
 __host__ __device__ constexpr uint32_t chunk_floats() { return kWarp * Rows<kDeg>::kC; }  // rows of one chunk
 
@@ -114,11 +106,6 @@ __device__ __forceinline__ void cp_async16_keep(float *dst, const float *src, ui
                  : "memory");
 }
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-// A hint to bring [p, p + bytes) into L2 (16-byte aligned, a multiple of 16 bytes); nothing
-// waits for it.
-__device__ __forceinline__ void prefetch_l2(const void *p, uint32_t bytes) {
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
-}
 
 struct Params {
     const qsdvr_ray_info *rays;
@@ -505,6 +492,8 @@ __device__ __forceinline__ uint32_t chunk_terms(const Params &p, float s1, uint3
 // such latency; with the two z planes loaded one after the other it waited two: 65536 rays at 128^3
 // fp32 degree 2 (train) 0.789 -> 0.750 ms, degree 3 (8192 rays, autograd) 0.410 -> 0.390, 256^3 bf16
 // degree 3 2.18 -> 2.15, 384^3 frame 5.39 -> 5.27 ms, its proposal form 1.70 -> 1.69.
+// (An L2 prefetch of the later steps' rows paid while a step waited twice; now it costs: 64^3 53.7 us
+// with and 51.3 without, 256^3 fp32 degree 2 1.568 and 1.556 ms.)
 template <typename S, int kDeg, bool kWide>
 __device__ __forceinline__ void gather_rows(const Params &p, float *tile, uint32_t shaded, int lane, float *to_slot) {
     using GL = GatherLanes<S, kDeg>;
@@ -617,22 +606,6 @@ __device__ __forceinline__ void eval_chunk(const Params &p, uint32_t r, f3 o, f3
                       : (uint32_t)s.cr.cx + (uint32_t)s.cr.cy * R1 + (uint32_t)s.cr.cz * (R1 * R1);
     if (shaded == 0) return;  // no sample of the chunk has a colour
     const int q = lane % kL;
-    const uint32_t sy = R1, sz = R1 * R1;
-    [[maybe_unused]] const uint64_t nv = (uint64_t)R1 * R1 * R1;  // vertex rows
-#if QSDVR_GATHER_PREFETCH
-    if constexpr (QSDVR_GATHER_PREFETCH == 2 || kDeg == 2) {
-        // samples of the gather's first round of loads (issued right below) are not prefetched
-        constexpr int kRound = GatherLanes<S, kDeg>::kPerStep * kGatherUnroll;
-        if (!from_slot && s.shaded && lane >= kRound) {
-            constexpr uint32_t kPair = 2u * kC * sizeof(S);  // rows v and v + 1 are adjacent
-            const S *base = static_cast<const S *>(p.data);
-            const uint32_t pv[4] = {s.vbase, s.vbase + sy, s.vbase + sz, s.vbase + sz + sy};
-#pragma unroll
-            for (int t = 0; t < 4; ++t)
-                prefetch_l2(QSDVR_AT(base, (uint64_t)kC * pv[t], 2 * kC, (uint64_t)kC * nv), kPair);
-        }
-    }
-#endif
     if (from_slot) {
         // rows stashed by the forward, one row per kL lanes per step, copied into the tile by
         // asynchronous 16-byte copies that are all in flight at once (one L2 round trip per
