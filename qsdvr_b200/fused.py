@@ -175,12 +175,9 @@ def ray_order(rays, origin, direction, interval, tlist=None) -> torch.Tensor:
     order = torch.empty(n, dtype=torch.int32, device=dev)
     if n == 0:
         return order
-    need = int(_lib.lib().qsdvr_ray_order_workspace_size(n))
-    key = (dev, "order")
-    ws = _workspaces.get(key)
-    if ws is None or ws.numel() < need:
-        ws = torch.empty(need, dtype=torch.uint8, device=dev)
-        _workspaces[key] = ws
+    # histogram and ranks of this call alone: calls on other streams or threads have their own, and the
+    # allocator gives the memory to later work of this stream only
+    ws = torch.empty(int(_lib.lib().qsdvr_ray_order_workspace_size(n)), dtype=torch.uint8, device=dev)
     if tlist is None:
         launch(dev, "qsdvr_ray_order", _ptr(rays), _ptr(origin), _ptr(direction), n, float(interval), _ptr(order),
                ws.data_ptr(), ws.numel())
