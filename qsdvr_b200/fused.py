@@ -50,19 +50,14 @@ _lib.extra_signatures({
     "qsdvr_render_forward_bricks": [ctypes.POINTER(RenderArgs), P],
 }, {"qsdvr_render_workspace_size": [ctypes.POINTER(RenderArgs)], "qsdvr_ray_order_workspace_size": [U32]})
 
-_workspaces: dict = {}
-
 
 def workspace(device, args: "RenderArgs") -> torch.Tensor:
-    """A cached workspace for the persistent kernels on ``device`` (one per device and
-    kernel configuration; launches on one stream never overlap, so it can be reused)."""
-    key = (device, args.mode, args.storage, args.transmittance, args.sh_degree)
+    """A workspace for one launch of the persistent kernels with ``args`` on ``device``'s current
+    stream.  The ray counter, the loss's partial sums, the row stash and the copies of a separable
+    gradient are in it, so launches that may overlap need one each: it comes from the caching
+    allocator at every call, which hands the memory on in the order of the stream."""
     need = int(_lib.lib().qsdvr_render_workspace_size(ctypes.byref(args)))
-    ws = _workspaces.get(key)
-    if ws is None or ws.numel() < need:
-        ws = torch.empty(need, dtype=torch.uint8, device=device)
-        _workspaces[key] = ws
-    return ws
+    return torch.empty(need, dtype=torch.uint8, device=device)
 
 
 def _ptr(t):
@@ -151,8 +146,8 @@ def make_args(rays, origin, direction, sdf_grid, data, reso, interval, k, mode="
         a.order = order.data_ptr()
     if persistent and n:
         with on_device(dev):
-            ws = workspace(dev, a)
-        a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
+            a.scratch = workspace(dev, a)  # kept as long as the arguments that point to it
+        a.workspace, a.workspace_bytes = a.scratch.data_ptr(), a.scratch.numel()
     return a
 
 

@@ -1,6 +1,6 @@
-"""Modules of different configuration that render on two streams at once: each gets the colours of
-its own single-stream run bit for bit, and its gradients up to the order of the float atomics (1e-5
-of the largest entry)."""
+"""Renders that share a device.  Modules of different configuration on two streams at once: each gets
+the colours of its own single-stream run bit for bit, and its gradients up to the order of the float
+atomics (1e-5 of the largest entry).  A captured step and later renders: the step's replay."""
 import pytest
 import torch
 
@@ -58,3 +58,43 @@ def test_two_modules_on_two_streams():
             assert torch.equal(g[0], w[0])
             for a, b in zip(g[1:], w[1:]):
                 assert rel_err(a.cpu(), b.cpu()) < 1e-5
+
+
+def test_captured_step_outlives_larger_renders():
+    """A captured training step replays the same colours and loss after separable models with larger
+    workspaces have rendered and the allocator's free memory has been given back and overwritten."""
+    from qsdvr_b200 import fused
+
+    R, interval = 64, 4.0 / 128
+    rays, o, d = _batches(R, interval)[0]
+    m = _models(R, interval)[0]
+    target = torch.rand((rays.shape[0], 3), generator=torch.Generator().manual_seed(1)).to(DEV)
+    sg, dg = torch.zeros_like(m.sdfGrid), torch.zeros_like(m.renderData)
+    loss = torch.zeros(1, device=DEV)
+
+    def step():
+        loss.zero_()
+        order = fused.ray_order(rays, o, d, interval)
+        return fused.render_train(target, rays, o, d, m.sdfGrid.detach(), m.renderData.detach(), R, interval, 5.0, sg, dg,
+                                  "fixed", loss=loss, order=order)[0]
+
+    want, want_loss = step().clone(), loss.item()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        color = step()
+    for big in (96, 160):
+        sep = fused.SeparableRenderGrid(big, interval=interval)
+        sep.train_step(target, rays, o, d)
+        del sep
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    filled = torch.full((1 << 28,), 0xFF, dtype=torch.uint8, device=DEV)
+    color.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(color, want)
+    # the same positive terms in another order, each sum of at most 512 (a warp), 128 and 6 additions
+    assert abs(loss.item() - want_loss) <= 2 * (512 + 128 + 6) * 2.0 ** -24 * want_loss
+    assert bool((filled == 0xFF).all())
