@@ -7,14 +7,14 @@ tables to the host after RayCut and back on every call).
 """
 from __future__ import annotations
 
-import ctypes
 import struct
 import zlib
 
 import numpy as np
 import torch
 
-from . import _lib, qsdvr
+from . import qsdvr
+from ._lib import launch
 from .qsdvr import CameraArgs
 
 
@@ -84,14 +84,16 @@ class Camera:
 
 
 def gather_rays(pixels: torch.Tensor, rays, origin, direction):
-    """(rays, origin, direction) of the listed pixels (int64 indices), one launch."""
+    """(rays, origin, direction) of the listed pixels (int64 indices into the per-pixel tables rays
+    int32 [P,4], origin and direction float32 [P,3]), one launch."""
     n, dev = pixels.numel(), rays.device
+    P = qsdvr._rays(rays, dev)
+    qsdvr._check(pixels, "pixels", torch.int64, dev, (n,))
+    for t, nm in ((origin, "origin"), (direction, "direction")):
+        qsdvr._check(t, nm, torch.float32, dev, (P, 3))
     out = (torch.empty((n, 4), dtype=torch.int32, device=dev), torch.empty((n, 3), dtype=torch.float32, device=dev),
            torch.empty((n, 3), dtype=torch.float32, device=dev))
-    with torch.cuda.device(dev):
-        _lib.call("qsdvr_gather_rays", ctypes.c_void_p(pixels.data_ptr()), n, rays.shape[0],
-                  *(ctypes.c_void_p(t.data_ptr()) for t in (rays, origin, direction, *out)),
-                  ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream))
+    launch(dev, "qsdvr_gather_rays", pixels.data_ptr(), n, P, *(t.data_ptr() for t in (rays, origin, direction, *out)))
     return out
 
 
