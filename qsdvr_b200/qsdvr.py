@@ -265,9 +265,10 @@ def LayerToGridForward(out, xLayer, yLayer, zLayer, offset):
         _check(t, nm, torch.float32, cuda=False)
     with on_device(dev):
         if not any(t.is_cuda or t.is_pinned() for t in (xLayer, yLayer, zLayer, offset)):
-            # pageable host layers (the reference's) cross in one copy instead of four
+            # pageable host layers (the reference's) cross in one copy instead of four; CUDA has staged it
+            # when the call returns, which does not wait for the stream
             x, y, z, off = torch.cat([xLayer.reshape(-1), yLayer.reshape(-1), zLayer.reshape(-1),
-                                      offset.reshape(-1)[:4]]).to(dev).split((R, R, R, 4))
+                                      offset.reshape(-1)[:4]]).to(dev, non_blocking=True).split((R, R, R, 4))
         else:
             x, y, z = (t.to(dev, non_blocking=True) for t in (xLayer, yLayer, zLayer))
             off = offset.reshape(-1)[:4].to(dev, non_blocking=True).contiguous()
