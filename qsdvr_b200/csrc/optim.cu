@@ -232,10 +232,29 @@ __device__ __forceinline__ float4 half4(const F8 &r, int h) {
 }
 
 constexpr int kDenseThreads = 512;
+constexpr unsigned kDenseRest = 4;  // threads past the groups of 8
+
+// What is left after the last whole group of 8: a group of 4 by the first thread past the groups,
+// then single elements, one a thread.  (As a launch of its own, by one thread, it took 2 of the 14
+// us of a call over 3 to 100003 elements; without it 11.)
+template <bool kBf16Grad>
+__device__ __noinline__ void adam_rest(const AdamParams a, uint32_t k) {
+    if (k == 0 && (a.n & 4)) {
+        const uint64_t i = a.n / 8 * 2;
+        float4 p;
+        adam_group<kBf16Grad>(a, i, p, false);
+        if (a.copy) copy4(a, i, p);
+    }
+    if (k > 0 && k <= (uint32_t)(a.n & 3)) adam_tail<kBf16Grad>(a, (a.n & ~3ull) + k - 1);
+}
+
 template <bool kBf16Grad, bool kBf16State, bool kCells>
 __global__ void __launch_bounds__(kDenseThreads) adam_dense_kernel(const AdamParams a) {
     const uint64_t i = blockIdx.x * (uint64_t)kDenseThreads + threadIdx.x;
-    if (i >= a.n / 8) return;
+    if (i >= a.n / 8) {
+        if (!kCells && i - a.n / 8 < kDenseRest) adam_rest<kBf16Grad>(a, (uint32_t)(i - a.n / 8));
+        return;
+    }
     const F8 g = kBf16Grad ? ld8_bf16(a.grad, i) : ld8(a.grad + 8 * i);
     F8 p = ld8(a.param + 8 * i);
     F8 m = kBf16State ? ld8_bf16(a.m, i) : ld8(a.m + 8 * i), v = kBf16State ? ld8_bf16(a.v, i) : ld8(a.v + 8 * i);
@@ -270,18 +289,6 @@ __global__ void __launch_bounds__(kDenseThreads) adam_dense_kernel(const AdamPar
             copy4(a, 2 * i + 1, half4(p, 1));
         }
     }
-}
-
-// What is left after the last whole group of 8: a group of 4, then single elements (one thread).
-template <bool kBf16Grad>
-__global__ void adam_rest_kernel(const AdamParams a) {
-    if (a.n & 4) {
-        const uint64_t i = a.n / 8 * 2;
-        float4 p;
-        adam_group<kBf16Grad>(a, i, p, false);
-        if (a.copy) copy4(a, i, p);
-    }
-    for (uint64_t e = a.n & ~3ull; e < a.n; ++e) adam_tail<kBf16Grad>(a, e);
 }
 
 // QSDVR_ADAM_SDF_CELLS: the parameters are quadric cells [n/8][8] with an fp32 gradient; one
@@ -358,15 +365,11 @@ extern "C" int qsdvr_adam_step(const qsdvr_adam_args *args, cudaStream_t stream)
                              "qsdvr_adam_step: SDF cells need a multiple of 8 elements and a 16-byte aligned copy");
     }
     if (dense) {
-        const unsigned n = grid_for(args->count / 8, kDenseThreads);
+        const unsigned n = grid_for(args->count / 8 + (args->count % 8 ? kDenseRest : 0), kDenseThreads);
         auto run = [&](auto kernel) { kernel<<<n, kDenseThreads, 0, stream>>>(a); };
         if (cells) a.state_bf16 ? run(adam_dense_kernel<false, true, true>) : run(adam_dense_kernel<false, false, true>);
         else if (grad_bf16) a.state_bf16 ? run(adam_dense_kernel<true, true, false>) : run(adam_dense_kernel<true, false, false>);
         else a.state_bf16 ? run(adam_dense_kernel<false, true, false>) : run(adam_dense_kernel<false, false, false>);
-        if (args->count % 8) {
-            if (grad_bf16) adam_rest_kernel<true><<<1, 1, 0, stream>>>(a);
-            else adam_rest_kernel<false><<<1, 1, 0, stream>>>(a);
-        }
     } else if (cells) {
         unsigned cblocks = grid_for(args->count / 8, 256);
         if (cblocks > cap) cblocks = cap;
