@@ -34,6 +34,7 @@ struct AdamParams {
     bool zero_grad, skip_zero;
     bool state_bf16;  // m and v hold bf16 values, stochastically rounded after each update
     uint32_t seed;    // per-step seed of the stochastic rounding
+    bool rest_stays;  // an element whose gradient and moments are 0 keeps its parameter and its moments
 };
 
 // Stochastic rounding of the bf16 moments (QSDVR_ADAM_STATE_BF16).  Adam's second moment
@@ -203,7 +204,12 @@ __global__ void __launch_bounds__(256) adam_kernel(const AdamParams a) {
 // warp touches 1 KB each.  With 16-byte accesses in a grid-stride loop of 16 blocks per SM the
 // streams' requests were too small and too few: the 671 M parameters of a 256^3 model (21.5 GB)
 // took 3.79 ms; with 32-byte accesses 3.36 ms, and 3.12 ms (6.88 TB/s) without the loop (blocks of
-// 512; 3.13 ms of 256).
+// 512; 3.13 ms of 256).  These are the gradients and moments of a grid whose rows
+// have all been touched.  The square root and the divisions take several times their usual
+// instructions on operands of 0, which bound the step over untouched rows (gradient and moments 0).
+// Nothing changes there, so a thread whose 8 elements are such leaves them: 33.5 M elements, half of
+// the rows untouched, 183 -> 117 us, all of them 173 -> 76; 3.1 M of a small grid, which the kernel of
+// groups of 4 took 18.9 us for, 20.9 -> 11.4.
 struct F8 {
     float v[8];
 };
@@ -248,18 +254,9 @@ __device__ __noinline__ void adam_rest(const AdamParams a, uint32_t k) {
     if (k > 0 && k <= (uint32_t)(a.n & 3)) adam_tail<kBf16Grad>(a, (a.n & ~3ull) + k - 1);
 }
 
-template <bool kBf16Grad, bool kBf16State, bool kCells>
-__global__ void __launch_bounds__(kDenseThreads) adam_dense_kernel(const AdamParams a) {
-    const uint64_t i = blockIdx.x * (uint64_t)kDenseThreads + threadIdx.x;
-    if (i >= a.n / 8) {
-        if (!kCells && i - a.n / 8 < kDenseRest) adam_rest<kBf16Grad>(a, (uint32_t)(i - a.n / 8));
-        return;
-    }
-    const F8 g = kBf16Grad ? ld8_bf16(a.grad, i) : ld8(a.grad + 8 * i);
-    F8 p = ld8(a.param + 8 * i);
-    F8 m = kBf16State ? ld8_bf16(a.m, i) : ld8(a.m + 8 * i), v = kBf16State ? ld8_bf16(a.v, i) : ld8(a.v + 8 * i);
-#pragma unroll
-    for (int q = 0; q < 8; ++q) adam_one(p.v[q], g.v[q], m.v[q], v.v[q], a);
+// Parameters, moments and the gradient's zeros of group i of 8.
+template <bool kBf16Grad, bool kBf16State>
+__device__ __forceinline__ void store_dense(const AdamParams &a, uint64_t i, const F8 &p, const F8 &m, const F8 &v) {
     st8(a.param + 8 * i, p);
     if (kBf16State) {
         uint2 mr[2], vr[2];
@@ -280,6 +277,27 @@ __global__ void __launch_bounds__(kDenseThreads) adam_dense_kernel(const AdamPar
     if (a.zero_grad) {
         if (kBf16Grad) reinterpret_cast<uint4 *>(a.grad)[i] = make_uint4(0u, 0u, 0u, 0u);
         else st8(a.grad + 8 * i, F8{{0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f}});
+    }
+}
+
+template <bool kBf16Grad, bool kBf16State, bool kCells>
+__global__ void __launch_bounds__(kDenseThreads) adam_dense_kernel(const AdamParams a) {
+    const uint64_t i = blockIdx.x * (uint64_t)kDenseThreads + threadIdx.x;
+    if (i >= a.n / 8) {
+        if (!kCells && i - a.n / 8 < kDenseRest) adam_rest<kBf16Grad>(a, (uint32_t)(i - a.n / 8));
+        return;
+    }
+    const F8 g = kBf16Grad ? ld8_bf16(a.grad, i) : ld8(a.grad + 8 * i);
+    F8 p = ld8(a.param + 8 * i);
+    F8 m = kBf16State ? ld8_bf16(a.m, i) : ld8(a.m + 8 * i), v = kBf16State ? ld8_bf16(a.v, i) : ld8(a.v + 8 * i);
+    uint32_t bits = 0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+        bits |= __float_as_uint(g.v[q]) | __float_as_uint(m.v[q]) | __float_as_uint(v.v[q]);
+    if (bits != 0 || !a.rest_stays) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) adam_one(p.v[q], g.v[q], m.v[q], v.v[q], a);
+        store_dense<kBf16Grad, kBf16State>(a, i, p, m, v);
     }
     if (a.copy) {
         if (kCells) {  // the compensated cell form
@@ -349,6 +367,8 @@ extern "C" int qsdvr_adam_step(const qsdvr_adam_args *args, cudaStream_t stream)
     a.skip_zero = (args->flags & QSDVR_ADAM_SKIP_ZERO_GRAD) != 0;
     a.state_bf16 = (args->flags & QSDVR_ADAM_STATE_BF16) != 0;
     a.seed = mix32_host(args->step);
+    // p - step_size (0 / eps) is p, its sign of 0 included, for these
+    a.rest_stays = a.eps > 0.0f && isfinite(a.eps) && a.step_size >= 0.0f && isfinite(a.step_size);
     const uint64_t work = (args->count + 3) / 4;
     unsigned blocks = grid_for(work, 256);
     const unsigned cap = 148u * 16;  // a few waves of resident blocks, grid-stride beyond
