@@ -45,11 +45,7 @@ namespace {
 #ifndef QSDVR_FORWARD_MIN_BLOCKS
 #define QSDVR_FORWARD_MIN_BLOCKS 20
 #endif
-#ifndef QSDVR_GATHER_UNROLL
-#define QSDVR_GATHER_UNROLL 1
-#endif
 constexpr int kWarpsPerBlock = QSDVR_FUSED_WARPS;
-constexpr int kGatherUnroll = QSDVR_GATHER_UNROLL;
 constexpr int kThreads = kWarpsPerBlock * kWarp;
 // Per SH degree: channels per row (32 or 64), staged row stride (+4 floats keeps both the
 // row-wise and the lane-wise float4 accesses bank-conflict free), lanes per sample in the
@@ -179,23 +175,23 @@ struct Store<__nv_bfloat16> {
     }
 };
 
-// Lanes of the appearance gather: each lane takes 32 bytes of a vertex row per corner (8 fp32 or
-// 16 bf16 channels), so kLanes lanes cover one row and a warp instruction fetches kPerStep
-// samples' rows.  32-byte loads halve the gather's instructions per byte (loads, addresses,
-// weights), which the issue-bound frames feel: 384^3 frame 5.92 -> 5.36 ms, its proposal form
-// 1.79 -> 1.70 ms, fp32 degree 3 at 128^3 (autograd) 0.427 -> 0.407 ms; the fp32 degree-2 training
-// batches, which memory bounds, stay as they were.
-template <typename S, int kDeg>
+// Lanes of the appearance gather: each lane takes kBytes of a vertex row per corner, so kLanes
+// lanes cover one row and a warp instruction fetches kPerStep samples' rows.  With 32 bytes (8 fp32
+// or 16 bf16 channels) the gather has half the instructions per byte (loads, addresses, weights),
+// which the issue-bound frames feel: 384^3 frame 5.92 -> 5.36 ms, its proposal form 1.79 -> 1.70 ms,
+// fp32 degree 3 at 128^3 (autograd) 0.427 -> 0.407 ms; the fp32 degree-2 training batches, which
+// memory bounds, stay as they were.  The fp32 degree-2 forward takes 16 bytes (kVarRow16).
+template <typename S, int kDeg, int kBytes>
 struct GatherLanes {
     static constexpr int kC = ShLayout<kDeg>::kChannels;
-    static constexpr int kCh = 32 / (int)sizeof(S);  // channels per lane
+    static constexpr int kCh = kBytes / (int)sizeof(S);  // channels per lane
     static constexpr int kLanes = kC / kCh;
     static constexpr int kPerStep = kWarp / kLanes;
 };
 
 // 32 bytes at p: one load where the grid is 32-byte aligned, else two.
 template <bool kWide>
-__device__ __forceinline__ void ld32(const void *p, uint32_t (&r)[8]) {
+__device__ __forceinline__ void ld_row(const void *p, uint32_t (&r)[8]) {
     if (kWide) {
         asm("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
@@ -205,6 +201,13 @@ __device__ __forceinline__ void ld32(const void *p, uint32_t (&r)[8]) {
         r[0] = lo.x; r[1] = lo.y; r[2] = lo.z; r[3] = lo.w;
         r[4] = hi.x; r[5] = hi.y; r[6] = hi.z; r[7] = hi.w;
     }
+}
+
+// 16 bytes at p, which every grid is aligned for.
+template <bool>
+__device__ __forceinline__ void ld_row(const void *p, uint32_t (&r)[4]) {
+    const uint4 v = *static_cast<const uint4 *>(p);
+    r[0] = v.x; r[1] = v.y; r[2] = v.z; r[3] = v.w;
 }
 
 __device__ __forceinline__ void red_cell(float *g8, uint32_t cell, const float *g, uint64_t cells) {
@@ -254,6 +257,16 @@ __device__ __forceinline__ void sep_red(float4 *sg, uint32_t R, const CellPoint 
 constexpr int kVarSep = 1;    // separable SDF tables instead of the dense cell grid
 constexpr int kVarMerge = 2;  // same-cell merged appearance scatter
 constexpr int kVarNarrow = 4; // the plain kernel for an appearance grid that is not 32-byte aligned
+// The plain forward over fp32 degree-2 rows for batches of kRow16Rays rays and more: 16-byte loads,
+// eight lanes a row, two steps an iteration.  The gather holds 32 registers of loads instead of 64,
+// the kernel 80 instead of 96, so 24 warps an SM hide its latencies instead of 20: 65536 rays at
+// 256^3 522 -> 485 us (from a sample list 223 -> 204), at 128^3 424 -> 373, at 64^3 94 -> 85.  With
+// about as many rays as resident warps each ray's own chain counts, which the 32-byte form makes
+// shorter: 2048 rays at 256^3 49.8 us with 16 bytes and 48.7 with 32, 3000 rays 55.8 and 55.4, 4096
+// rays 60.1 and 61.5, 8192 rays 94.5 and 97.3.  bf16 rows (405 and 402 us) and the separable SDF (474
+// and 459) are better off with 32 bytes, and in the training passes the two forms tie.
+constexpr int kVarRow16 = 8;
+constexpr uint32_t kRow16Rays = 4096;
 
 template <typename S, int kVar>
 __device__ __forceinline__ void load_cell(const Params &p, const CellPoint &c, float *a) {
@@ -316,14 +329,14 @@ __device__ __forceinline__ void fma_bf8(uint4 r, float w, float *v) {
     for (int t = 0; t < 4; ++t) ffma2(v[2 * t], v[2 * t + 1], w, bf_lo(rv[t]), bf_hi(rv[t]));
 }
 
-// v = w * (the channels of 32 bytes r), or v += w * (...)
-template <typename S, bool kFirst>
-__device__ __forceinline__ void weigh32(const uint32_t (&r)[8], float w, float *v) {
+// v = w * (the channels of the 4 kN bytes r), or v += w * (...)
+template <typename S, bool kFirst, int kN>
+__device__ __forceinline__ void weigh_row(const uint32_t (&r)[kN], float w, float *v) {
 #pragma unroll
-    for (int t = 0; t < 8; t += sizeof(S) == 2 ? 1 : 2) {
+    for (int t = 0; t < kN; t += sizeof(S) == 2 ? 1 : 2) {
         // the next two channels: a pair of bf16 or two floats
         const float x0 = sizeof(S) == 2 ? bf_lo(r[t]) : __uint_as_float(r[t]);
-        const float x1 = sizeof(S) == 2 ? bf_hi(r[t]) : __uint_as_float(r[(t + 1) & 7]);
+        const float x1 = sizeof(S) == 2 ? bf_hi(r[t]) : __uint_as_float(r[(t + 1) & (kN - 1)]);
         float *o = v + (sizeof(S) == 2 ? 2 * t : t);
         if (kFirst) {
             o[0] = w * x0;
@@ -494,21 +507,21 @@ __device__ __forceinline__ uint32_t chunk_terms(const Params &p, float s1, uint3
 // degree 3 2.18 -> 2.15, 384^3 frame 5.39 -> 5.27 ms, its proposal form 1.70 -> 1.69.
 // (An L2 prefetch of the later steps' rows paid while a step waited twice; now it costs: 64^3 53.7 us
 // with and 51.3 without, 256^3 fp32 degree 2 1.568 and 1.556 ms.)
-template <typename S, int kDeg, bool kWide>
+template <typename S, int kDeg, int kBytes, bool kWide, int kSteps = 1>
 __device__ __forceinline__ void gather_rows(const Params &p, float *tile, uint32_t shaded, int lane, float *to_slot) {
-    using GL = GatherLanes<S, kDeg>;
+    using GL = GatherLanes<S, kDeg, kBytes>;
     constexpr int kC = GL::kC, kRow = Rows<kDeg>::kStride, kGL = GL::kLanes, kGPS = GL::kPerStep, kCh = GL::kCh;
-    constexpr int kRound = kGPS * kGatherUnroll;
-    constexpr uint32_t kRoundMask = kRound >= 32 ? 0xffffffffu : (1u << (kRound & 31)) - 1u;
+    constexpr int kRound = kGPS * kSteps;  // samples of an iteration
+    static_assert(kRound < kWarp);
     const uint32_t R1 = p.R + 1;
     const uint64_t dy = (uint64_t)kC * R1, dz = dy * R1;  // elements to the rows above in y and z
     [[maybe_unused]] const uint64_t ne = dz * R1;
     const int gq = lane % kGL;
 #pragma unroll 1
     for (int first = 0; first < kWarp; first += kRound) {
-        if (((shaded >> first) & kRoundMask) == 0) continue;  // warp-uniform
+        if (((shaded >> first) & ((1u << kRound) - 1u)) == 0) continue;  // warp-uniform
 #pragma unroll
-        for (int u = 0; u < kGatherUnroll; ++u) {
+        for (int u = 0; u < kSteps; ++u) {
             const int j = first + u * kGPS + lane / kGL;
             const float4 prm = ld4(tile + j * kRow + kC);
             const uint32_t vb = __float_as_uint(prm.x);
@@ -517,18 +530,18 @@ __device__ __forceinline__ void gather_rows(const Params &p, float *tile, uint32
             const S *d = static_cast<const S *>(p.data);
             float w[8], v[kCh];
             corner_weights(prm.y, prm.z, prm.w, w);
-            uint32_t c[8][8];  // all eight corners' loads are issued before the first is used
+            uint32_t c[8][kBytes / 4];  // all eight corners' loads are issued before the first is used
 #pragma unroll
             for (int h = 0; h < 2; ++h) {  // the corners of the lower and of the upper z plane
                 const uint64_t ez = h ? e + dz : e;
-                ld32<kWide>(QSDVR_AT(d, ez, kCh, ne), c[4 * h]);
-                ld32<kWide>(QSDVR_AT(d, ez + kC, kCh, ne), c[4 * h + 1]);
-                ld32<kWide>(QSDVR_AT(d, ez + dy, kCh, ne), c[4 * h + 2]);
-                ld32<kWide>(QSDVR_AT(d, ez + dy + kC, kCh, ne), c[4 * h + 3]);
+                ld_row<kWide>(QSDVR_AT(d, ez, kCh, ne), c[4 * h]);
+                ld_row<kWide>(QSDVR_AT(d, ez + kC, kCh, ne), c[4 * h + 1]);
+                ld_row<kWide>(QSDVR_AT(d, ez + dy, kCh, ne), c[4 * h + 2]);
+                ld_row<kWide>(QSDVR_AT(d, ez + dy + kC, kCh, ne), c[4 * h + 3]);
             }
-            weigh32<S, true>(c[0], w[0], v);
+            weigh_row<S, true>(c[0], w[0], v);
 #pragma unroll
-            for (int k = 1; k < 8; ++k) weigh32<S, false>(c[k], w[k], v);
+            for (int k = 1; k < 8; ++k) weigh_row<S, false>(c[k], w[k], v);
 #pragma unroll
             for (int t = 0; t < kCh; t += 4) {
                 const float4 q = make_float4(v[t], v[t + 1], v[t + 2], v[t + 3]);
@@ -633,13 +646,15 @@ __device__ __forceinline__ void eval_chunk(const Params &p, uint32_t r, f3 o, f3
         __syncwarp();
         // (both forms in one kernel cost the plain one 1 %, so its narrow form is an instance of
         // its own; the separable and the merged kernels choose at run time)
-        if constexpr (kVar == 0) {
-            gather_rows<S, kDeg, true>(p, tile, shaded, lane, to_slot);
+        if constexpr ((kVar & kVarRow16) != 0) {
+            gather_rows<S, kDeg, 16, false, 2>(p, tile, shaded, lane, to_slot);
+        } else if constexpr (kVar == 0) {
+            gather_rows<S, kDeg, 32, true>(p, tile, shaded, lane, to_slot);
         } else if constexpr (kVar == kVarNarrow) {
-            gather_rows<S, kDeg, false>(p, tile, shaded, lane, to_slot);
+            gather_rows<S, kDeg, 32, false>(p, tile, shaded, lane, to_slot);
         } else {
-            if (p.wide) gather_rows<S, kDeg, true>(p, tile, shaded, lane, to_slot);
-            else gather_rows<S, kDeg, false>(p, tile, shaded, lane, to_slot);
+            if (p.wide) gather_rows<S, kDeg, 32, true>(p, tile, shaded, lane, to_slot);
+            else gather_rows<S, kDeg, 32, false>(p, tile, shaded, lane, to_slot);
         }
         __syncwarp();
     }
@@ -1356,6 +1371,12 @@ void dispatch(const qsdvr_render_args *a, F &f) {
 template <int kPass, int kVar>
 constexpr int pass_variant() { return kPass == kForward ? (kVar & ~kVarMerge) : kVar; }
 
+// Whether a pass has a kVarRow16 instance beside kVar, whatever the grid's alignment.
+template <int kPass, typename S, int kDeg, int kVar>
+constexpr bool has_row16() {
+    return kPass == kForward && sizeof(S) == 4 && kDeg == 2 && (kVar == 0 || kVar == kVarNarrow);
+}
+
 // Persistent grid and workspace size for the current device: one block per resident slot
 // of the train kernel (the heaviest instantiation, which bounds the others).
 struct Layout {
@@ -1366,6 +1387,7 @@ struct Layout {
 
 struct Occupancy {
     int pass = kTrain;
+    uint32_t rays = 0;
     int per_sm = 0, train_per_sm = 0;
     size_t chunk_bytes = 0;
     cudaError_t err = cudaSuccess;
@@ -1374,9 +1396,12 @@ struct Occupancy {
         err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&train_per_sm, render_kernel<C, S, kTrain, L, D, V>, kThreads,
                                                             0);
         per_sm = train_per_sm;
-        if (err == cudaSuccess && pass == kForward)
-            err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                &per_sm, render_kernel<C, S, kForward, L, D, pass_variant<kForward, V>()>, kThreads, 0);
+        if (err == cudaSuccess && pass == kForward) {
+            auto kernel = render_kernel<C, S, kForward, L, D, pass_variant<kForward, V>()>;
+            if constexpr (has_row16<kForward, S, D, V>())
+                if (rays >= kRow16Rays) kernel = render_kernel<C, S, kForward, L, D, kVarRow16>;
+            err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, 0);
+        }
         if (err == cudaSuccess && pass == kBackward)
             err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, render_kernel<C, S, kBackward, L, D, V>,
                                                                 kThreads, 0);
@@ -1397,6 +1422,7 @@ Layout layout_for(const qsdvr_render_args *a, int pass = kTrain) {
     }
     Occupancy occ;
     occ.pass = pass;
+    occ.rays = a->ray_count;
     // the grid and the workspace do not depend on the grid's alignment: a size that was asked for
     // before the pointers were known stays right
     qsdvr_render_args variant = *a;
@@ -1421,7 +1447,10 @@ struct Launcher {
     cudaStream_t stream;
     template <bool C, typename S, bool L, int D, int V>
     void run() {
-        render_kernel<C, S, kPass, L, D, pass_variant<kPass, V>()><<<blocks, kThreads, 0, stream>>>(*p);
+        auto kernel = render_kernel<C, S, kPass, L, D, pass_variant<kPass, V>()>;
+        if constexpr (has_row16<kPass, S, D, V>())
+            if (p->n >= kRow16Rays) kernel = render_kernel<C, S, kPass, L, D, kVarRow16>;
+        kernel<<<blocks, kThreads, 0, stream>>>(*p);
     }
 };
 
