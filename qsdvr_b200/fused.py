@@ -50,13 +50,23 @@ _lib.extra_signatures({
     "qsdvr_render_forward_bricks": [ctypes.POINTER(RenderArgs), P],
 }, {"qsdvr_render_workspace_size": [ctypes.POINTER(RenderArgs)], "qsdvr_ray_order_workspace_size": [U32]})
 
+_workspace_bytes: dict = {}  # per device and kernel configuration
+
 
 def workspace(device, args: "RenderArgs") -> torch.Tensor:
     """A workspace for one launch of the persistent kernels with ``args`` on ``device``'s current
     stream.  The ray counter, the loss's partial sums, the row stash and the copies of a separable
     gradient are in it, so launches that may overlap need one each: it comes from the caching
-    allocator at every call, which hands the memory on in the order of the stream."""
-    need = int(_lib.lib().qsdvr_render_workspace_size(ctypes.byref(args)))
+    allocator at every call, which hands the memory on in the order of the stream.  Its size is the
+    library's answer for the configuration, asked once."""
+    key = (device, args.mode, args.storage, args.transmittance, args.sh_degree, args.merge_scatter,
+           args.reso if args.sdf_layers else 0)
+    need = _workspace_bytes.get(key)
+    if not need:  # not asked yet, or the query failed (0)
+        if len(_workspace_bytes) >= 1024:
+            _workspace_bytes.clear()
+        with on_device(device):
+            need = _workspace_bytes[key] = int(_lib.lib().qsdvr_render_workspace_size(ctypes.byref(args)))
     return torch.empty(need, dtype=torch.uint8, device=device)
 
 
@@ -145,9 +155,8 @@ def make_args(rays, origin, direction, sdf_grid, data, reso, interval, k, mode="
             raise ValueError(f"order must be a contiguous int32 [N] permutation on {dev}")
         a.order = order.data_ptr()
     if persistent and n:
-        with on_device(dev):
-            a.scratch = workspace(dev, a)  # kept as long as the arguments that point to it
-        a.workspace, a.workspace_bytes = a.scratch.data_ptr(), a.scratch.numel()
+        ws = a.scratch = workspace(dev, a)  # kept as long as the arguments that point to it
+        a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
     return a
 
 
