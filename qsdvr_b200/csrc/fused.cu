@@ -7,11 +7,10 @@
 //   * lane i owns render sample i of the chunk: its positions (bit-exact with
 //     GenerateRayPoints), quadric cells, SDF values, normal, alpha and shading;
 //   * the 32-channel appearance rows are gathered with 32-byte loads by groups of 4 lanes
-//     (8 floats each) or 2 lanes (16 bf16 each), so every load covers whole 128-byte
-//     (64-byte bf16) vertex rows, interpolated and staged in a per-warp shared-memory
-//     tile [32][36] floats
-//     (row stride 36 keeps both the row-wise and the lane-wise float4 accesses
-//     conflict-free);
+//     (8 floats each) or 2 lanes (16 bf16 each; the fp32 forward of larger batches takes 16-byte
+//     loads and 8 lanes), so every load covers whole 128-byte (64-byte bf16) vertex rows,
+//     interpolated and staged in a per-warp shared-memory tile [32][36] floats
+//     (row stride 36 keeps the lane-wise float4 accesses free of bank conflicts);
 //   * transmittance is an exclusive prefix product (or a compensated prefix sum of
 //     log(1 - alpha)) by warp shuffles, carried across chunks;
 //   * the backward walks the chunks in reverse, carrying the suffix state, and
@@ -47,9 +46,10 @@ namespace {
 #endif
 constexpr int kWarpsPerBlock = QSDVR_FUSED_WARPS;
 constexpr int kThreads = kWarpsPerBlock * kWarp;
-// Per SH degree: channels per row (32 or 64), staged row stride (+4 floats keeps both the
-// row-wise and the lane-wise float4 accesses bank-conflict free), lanes per sample in the
-// gather/scatter (one float4 each) and samples per warp instruction.
+// Per SH degree: channels per row (32 or 64), staged row stride (+4 floats keeps the lane-wise float4
+// accesses free of bank conflicts, and the row-wise ones of a float4 a lane; of the gather's stores,
+// 8 or 16 floats a lane, those of the degree-3 rows conflict in pairs), lanes per sample in the
+// scatter (one float4 each) and samples per warp instruction.
 template <int kDeg>
 struct Rows {
     static constexpr int kC = ShLayout<kDeg>::kChannels;
@@ -58,17 +58,17 @@ struct Rows {
     static constexpr int kPerStep = kWarp / kLanes;
 };
 constexpr uint32_t kMaxChunks = 256;  // render samples per ray <= 8192
-// Each staged tile row carries 4 floats of padding (the row stride keeps the row-wise and
-// lane-wise float4 accesses bank-conflict free); the gather and the scatter keep there the
+// Each staged tile row carries 4 floats of padding; the gather and the scatter keep there the
 // sample's (base vertex, wx, wy, wz), the vertex kNoVertex for a sample without a row, so a
 // step reads one sample's parameters with one 16-byte shared load instead of 5 shuffles.
 constexpr uint32_t kNoVertex = 0xffffffffu;
 constexpr uint32_t kLossParts = 32;  // word offset of the loss's partial sums behind the ray counter
 
 enum Pass { kForward = 0, kBackward = 1, kTrain = 2 };
-// Resident one-warp blocks per SM that each pass is compiled for.  The forward's 20 are what its
-// shared memory allows; compiled for 16 it took up to 126 registers and lost four of them (a 384^3
-// frame 7.0 instead of 6.0 ms).
+// Resident one-warp blocks per SM that each pass is compiled for.  Compiled for 16 the forward took up
+// to 126 registers and lost blocks to them: a 384^3 frame of degree 3 7.0 instead of 6.0 ms with 20
+// (its shared memory, 9 KB a block, allows 24), 65536 fp32 degree-2 rays at 256^3 515 instead of 485
+// us (4.6 KB a block; its 16-byte form takes 80 registers, which give 24).
 constexpr int min_blocks(int pass) { return pass == kForward ? QSDVR_FORWARD_MIN_BLOCKS : QSDVR_FUSED_MIN_BLOCKS; }
 
 // Persistent train mode: each warp stashes the interpolated rows of the kSlotChunks chunks
@@ -506,7 +506,9 @@ __device__ __forceinline__ uint32_t chunk_terms(const Params &p, float s1, uint3
 // fp32 degree 2 (train) 0.789 -> 0.750 ms, degree 3 (8192 rays, autograd) 0.410 -> 0.390, 256^3 bf16
 // degree 3 2.18 -> 2.15, 384^3 frame 5.39 -> 5.27 ms, its proposal form 1.70 -> 1.69.
 // (An L2 prefetch of the later steps' rows paid while a step waited twice; now it costs: 64^3 53.7 us
-// with and 51.3 without, 256^3 fp32 degree 2 1.568 and 1.556 ms.)
+// with and 51.3 without, 256^3 fp32 degree 2 1.568 and 1.556 ms.  The fp32 degree-2 forward in
+// 16-byte pieces: 65536 rays at 256^3 479 us with and 485 without, at 128^3 385 and 373, at 64^3 93 and
+// 85; bf16 forward and training at 256^3 the same either way.)
 template <typename S, int kDeg, int kBytes, bool kWide, int kSteps = 1>
 __device__ __forceinline__ void gather_rows(const Params &p, float *tile, uint32_t shaded, int lane, float *to_slot) {
     using GL = GatherLanes<S, kDeg, kBytes>;

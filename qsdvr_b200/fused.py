@@ -276,11 +276,17 @@ def render_train(target, rays, origin, direction, sdf_grid, data, reso, interval
 
 def gradient_order(rays, origin, direction, interval, data, reso):
     """``ray_order`` of a batch that is about to be rendered with gradients where that pays, else
-    None.  The order costs about 17 us and shares rows and gradient lines between neighbouring
-    rays in L2, so it pays for grids well above L2 (64 MB: at 64^3 the rows stay in L2 either way)
-    and batches dense enough to have such neighbours.  Forward + backward at 128^3, fp32 degree
-    2: 8192 rays 270 us in batch order, 283 ordered; 16384 rays 461 / 437; 65536 rays 1624 /
-    1277.  At 256^3: 16384 rays 572 / 585, 32768 rays 1062 / 1040, 65536 rays 2051 / 1951."""
+    None.  The order costs about 20 us and shares rows and gradient lines between neighbouring
+    rays in L2, so it pays where the rows and their fp32 gradients do not both stay there (rows of
+    64 MB and more: with as many bytes of gradients they fill L2's 126 MB) and in batches dense
+    enough to have such neighbours.  A module's step (forward, loss, backward), in batch order /
+    ordered, us; fp32 degree 2, 64^3 (34 MB): 16384 rays 237 / 264, 65536 rays 540 / 552; 80^3 (65
+    MB): 276 / 280, 771 / 691; 96^3 (111 MB): 357 / 349, 1072 / 856; 128^3: 8192 rays 345 / 359,
+    16384 rays 527 / 501, 65536 rays 1608 / 1257; 224^3: 16384 rays 824 / 830, 32768 rays 1294 / 1244.
+    Degree 3, 64^3 (67 MB): 16384 rays 290 / 298, 65536 rays 831 / 788; 128^3: 781 / 752, 2453 /
+    1970.  bf16 degree 2, 112^3 (88 MB): 402 / 398, 1229 / 1035; 256^3: 16384 rays 930 / 933, 32768
+    rays 1392 / 1341; bf16 degree 3, 80^3 (65 MB): 363 / 366, 1092 / 1004; 256^3: 32768 rays 2042 /
+    2025."""
     n = rays.shape[0]
     if n < 16384 or 2 * n < int(reso) ** 2 or data.numel() * data.element_size() < 64 << 20:
         return None
