@@ -66,9 +66,9 @@ constexpr uint32_t kLossParts = 32;  // word offset of the loss's partial sums b
 
 enum Pass { kForward = 0, kBackward = 1, kTrain = 2 };
 // Resident one-warp blocks per SM that each pass is compiled for.  Compiled for 16 the forward took up
-// to 126 registers and lost blocks to them: a 384^3 frame of degree 3 7.0 instead of 6.0 ms with 20
-// (its shared memory, 9 KB a block, allows 24), 65536 fp32 degree-2 rays at 256^3 515 instead of 485
-// us (4.6 KB a block; its 16-byte form takes 80 registers, which give 24).
+// to 126 registers and lost blocks to them: a 384^3 frame of degree 3 7.0 ms, and 6.0 with the 96
+// registers that give 20; 65536 fp32 degree-2 rays at 256^3 515 us, and 485 (their 16-byte form takes 80
+// registers, which give 24).
 constexpr int min_blocks(int pass) { return pass == kForward ? QSDVR_FORWARD_MIN_BLOCKS : QSDVR_FUSED_MIN_BLOCKS; }
 
 // Persistent train mode: each warp stashes the interpolated rows of the kSlotChunks chunks
